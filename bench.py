@@ -113,6 +113,10 @@ def issue_ops_per_labeling(desc: str, d: int, cols: int) -> tuple[int, str]:
              .replace("int8x4 words", "int8x4_words").split() if "=" in kv)
     if desc.startswith("table") and "int32_words" in f:
         D, wb, wa = int(f["D"]), int(f["int32_words"]), int(f["int8x4_words"])
+        if int(f.get("half", 0)) > 0:
+            # two columns per word: a pair maximum and a multiply-add
+            words = (cols + 1) // 2
+            return 2 * D * words, f"2 slots x D={D} x {words} int16x2 words (pair maximum, multiply-add), unpadded"
         if int(f.get("split", 0)) > 0:
             # column split: the words of the actual columns (the padding to
             # S x PW words is not counted as work)
@@ -712,11 +716,14 @@ def run_batch(args) -> None:
     t0 = time.perf_counter()
     b = ld.Batch(mats, ds, opts=opts, autotune=True)
     create_s = time.perf_counter() - t0
-    # int32 issue slots: one sad (2 slots) per column per sum vector (all of
-    # this workload's sums need 32-bit lanes) per labeling the kernels
-    # evaluate (d = 3: label symmetry skips about half)
+    # int32 issue slots per labeling the kernels evaluate (d = 3: label
+    # symmetry skips about half): two columns per word, a pair maximum and a
+    # multiply-add per two columns and sum vector; 32-bit lanes, one sad (2
+    # slots) per column and sum vector
     evaluated = b.evaluated()
-    slots = sum(2 * dd * m.shape[1] * int(e) for dd, m, e in zip(ds, mats, evaluated))
+    half = all("int32=0 " in c for c in b.describe().split("; ")[1:])
+    slots = sum((2 * ((m.shape[1] + 1) // 2) if half else 2 * m.shape[1]) * dd * int(e)
+                for dd, m, e in zip(ds, mats, evaluated))
     n_eval = int(evaluated.sum())
     for _ in range(args.warmup):
         v0, g0, _ = b.solve()
@@ -806,8 +813,8 @@ def run_batch(args) -> None:
                 "d2h_bytes_per_step": len(mats) * 16, "s_per_step": statistics.mean(e2e)},
         "roofline": {"bound": "int32", "achieved": achieved / 1e12, "peak": peak_ops / 1e12, "unit": "Tops/s",
                      "frac": achieved / peak_ops, "traffic": None, "ops_per_labeling": slots / max(n_eval, 1),
-                     "note": "2 int32 issue slots (one sad) per column per sum vector per evaluated labeling, unpadded "
-                             "columns, averaged over the batch; peak = int32 add/xor microbenchmark measured "
+                     "note": f"2 int32 issue slots per {'two columns' if half else 'column'} per sum vector per "
+                             "evaluated labeling, unpadded columns, averaged over the batch; peak = int32 add/xor microbenchmark measured "
                              "in this run"},
         # per replay: one persistent kernel per lane class, the fold, and the own plans' kernels
         "gpu_launches": len(ms) * (int(desc.split(" classes")[0].split()[-1]) + 1

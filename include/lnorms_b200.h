@@ -52,7 +52,8 @@ typedef struct {
                               a bound or by label symmetry)                        */
     float kernel_ms;       /* device time of the solve's launches (CUDA events)     */
     int32_t kernel_kind;   /* LD_KERNEL_* actually used                             */
-    int32_t lane_bits;     /* 8, 16, 32 or 64: arithmetic lane width used           */
+    int32_t lane_bits;     /* 8, 32 or 64: arithmetic lane width used (32: also two
+                              columns per 32-bit word where they fit)               */
     uint64_t h2d_bytes;    /* host-to-device bytes this solve copied                */
     uint64_t d2h_bytes;    /* device-to-host bytes this solve copied                */
     uint64_t evaluated;    /* labelings the kernels computed a value for (fewer
@@ -101,9 +102,11 @@ typedef struct {
     int32_t paired_walks;       /* table kernel, d <= 3: 0 = two high indices per
                                    thread against each table read when every
                                    thread has at least two walks; -1 = one   */
-    int32_t pack16;             /* table kernel: 0 = keep two running maxima in
-                                   one word (16 bits each) when every value is
-                                   below 65536; -1 = one maximum per word    */
+    int32_t pack16;             /* table kernels and batches: 0 = 16-bit forms
+                                   where the values fit: two running maxima in
+                                   one word when every value is below 65536,
+                                   and (d <= 3, columns that need 32-bit lanes
+                                   otherwise) two columns per word; -1 = none */
     int32_t walk_fetch;         /* table kernel: 0 = warps fetch walks from a
                                    counter as they finish (balanced); -1 =
                                    every thread takes a fixed share         */

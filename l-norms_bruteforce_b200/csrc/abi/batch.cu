@@ -28,6 +28,7 @@ using namespace ldsolve;
 #include <tuple>
 
 #include "../kernels/batch_kernel.cuh"
+#include "../kernels/half_kernel.cuh"
 #include "device_guard.h"
 
 namespace {
@@ -38,6 +39,7 @@ constexpr int kTpbChoices[kTpbN] = {64, 128};
 
 struct BatchClass {
   int D = 0, WB = 0, WA = 0;
+  int HW = 0;                     // two columns per word: words per vector (WB = 2 HW), else 0
   const void* kfn = nullptr;
   size_t smem = 0;
   int bps = 1;                    // resident CTAs per SM at tpb threads (plain instance)
@@ -64,7 +66,7 @@ struct BatchClass {
   cudaEvent_t done = nullptr;
 };
 
-// autotuner cache: (D, WB, WA, log2 of the mean walks per problem, batch_split option)
+// autotuner cache: (D, WB, WA or -1 for two columns per word, log2 of the mean walks per problem, batch_split option)
 //   -> (wpt, grid fraction, split, threads per CTA, low-row shift)
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int, int>, std::tuple<int, double, bool, int, int>> g_tune;
@@ -157,7 +159,7 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
   std::vector<std::vector<char>> images(count);
   std::vector<Choice> pch(count);                        // lane layout per class matrix
   std::vector<int> kmax(count, -1);                      // the largest low-row count that fits
-  std::map<std::tuple<int, int, int>, int> class_of;
+  std::map<std::tuple<int, int, int, int>, int> class_of;
   b->hprob.resize(count);
   // walks of matrix p at low-row count k: whole high indices, at most about
   // 2^16 walks (enough chunks to spread one large matrix); fw = walked digits
@@ -193,11 +195,25 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
       }
     }
     std::vector<char>& img = images[p];
-    img.assign(768 + align256((size_t)R * WT * 4), 0);
-    pack_row(tot.data(), ch, (uint32_t*)(img.data() + 0));
-    pack_row(h0.data(), ch, (uint32_t*)(img.data() + 256));
-    pack_row(tb.data(), ch, (uint32_t*)(img.data() + 512));
-    for (int i = 0; i < R; ++i) pack_row(a + (size_t)i * C, ch, (uint32_t*)(img.data() + 768) + (size_t)i * WT);
+    const int vw = ch.HW > 0 ? half_vector_words(ch.HW, 1) : WT;
+    img.assign(768 + align256((size_t)R * vw * 4), 0);
+    auto words = [&](size_t off) { return (uint32_t*)(img.data() + off); };
+    long long value_bias = 0;
+    if (ch.HW > 0) {
+      HalfLayout lay;
+      half_layout(a, R, C, d, marg, k, ch.HW, 1, &lay);   // fits: checked when the class was chosen
+      half_pack(tot.data(), lay.beta.data(), C, ch.HW, 1, words(0));
+      half_pack(h0.data(), lay.beta.data(), C, ch.HW, 1, words(256));
+      half_pack(tb.data(), lay.beta.data(), C, ch.HW, 1, words(512));
+      words(512)[ch.HW + 1] = lay.seed[0];
+      for (int i = 0; i < R; ++i) half_pack(a + (size_t)i * C, nullptr, C, ch.HW, 1, words(768) + (size_t)i * vw);
+      value_bias = lay.value_bias;
+    } else {
+      pack_row(tot.data(), ch, words(0));
+      pack_row(h0.data(), ch, words(256));
+      pack_row(tb.data(), ch, words(512));
+      for (int i = 0; i < R; ++i) pack_row(a + (size_t)i * C, ch, words(768) + (size_t)i * WT);
+    }
     ld::BatchProblem bp = b->hprob[p];   // keeps the device pointers
     bp.R = R; bp.k = k; bp.B = B; bp.fw = fw;
     bp.walk_len = ipow(base, fw);
@@ -212,7 +228,7 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
       run = walks[p];
     }
     b->evaluated[p] = (unsigned long long)run * bp.walk_len * (unsigned long long)B;
-    bp.value_offset = kh + kl;
+    bp.value_offset = kh + kl - value_bias;
     b->hprob[p] = bp;
   };
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -253,7 +269,19 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
           // with all-int32 lanes the column order is the identity and every column is wide
         }
         c.WT = round4(c.WB + c.WA);
-        if (!ld::batch_kernel_ptr(d, c.WB, c.WA) || B * (unsigned long long)(d * c.WT) > 4096ull) continue;
+        // two columns per word when the values fit at every low-row count the
+        // tuner may try; the table then has room for about one low row more
+        c.HW = 0;
+        if (c.WB > 0 && o.batch_split <= 0 && o.pack16 >= 0 && o.lane_bits == 0 &&
+            B * (unsigned long long)ld::half_entry_words(d, c.WB / 2) <= 4096ull) {
+          HalfLayout lay;
+          bool fits = true;
+          for (int q = kk; q >= std::max(0, kk - 2) && fits; --q)
+            fits = half_layout(a, R, C, d, marg, q, c.WB / 2, 1, &lay);
+          if (fits) c.HW = c.WB / 2;
+        }
+        if (!ld::batch_kernel_ptr(d, c.WB, c.WA) || (c.HW == 0 && B * (unsigned long long)(d * c.WT) > 4096ull))
+          continue;
         if (c.WB > 0) {      // re-pack every column as int32 (table_config may have put some in int8)
           c.order.clear();
           for (int l = 0; l < C; ++l) c.order.push_back(l);
@@ -277,7 +305,7 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
       b->evaluated[p] = plan_evaluated(plan);
       continue;
     }
-    const auto key = std::make_tuple(d, ch.WB, ch.WA);
+    const auto key = std::make_tuple(d, ch.WB, ch.WA, ch.HW);
     auto it = class_of.find(key);
     int ci;
     if (it == class_of.end()) {
@@ -285,8 +313,9 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
       class_of[key] = ci;
       BatchClass bc;
       bc.D = d; bc.WB = ch.WB; bc.WA = ch.WA;
-      bc.kfn = ld::batch_kernel_ptr(d, ch.WB, ch.WA);
-      if (ch.WA == 0 && o.batch_split >= 0) bc.kfn_split = ld::batch_split_kernel_ptr(d, ch.WB);
+      bc.HW = ch.HW;
+      bc.kfn = ch.HW > 0 ? ld::batch_half_kernel_ptr(d, ch.HW) : ld::batch_kernel_ptr(d, ch.WB, ch.WA);
+      if (ch.HW == 0 && ch.WA == 0 && o.batch_split >= 0) bc.kfn_split = ld::batch_split_kernel_ptr(d, ch.WB);
       b->classes.push_back(bc);
     } else {
       ci = it->second;
@@ -306,7 +335,8 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
     c.smem_split = 0;
     for (int p : c.probs) {
       const ld::BatchProblem& bp = b->hprob[p];
-      c.smem = std::max(c.smem, (size_t)ld::table_smem_words(c.D, pch[p].WT, bp.R, bp.B) * 4);
+      c.smem = std::max(c.smem, (size_t)(c.HW > 0 ? ld::half_region_words(c.D, c.HW, bp.R, bp.B)
+                                                  : ld::table_smem_words(c.D, pch[p].WT, bp.R, bp.B)) * 4);
       if (c.kfn_split)
         c.smem_split = std::max(c.smem_split, (size_t)ld::batch_split_smem_words(c.D, c.WB, bp.R, bp.B) * 4);
     }
@@ -421,6 +451,7 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
   // once; the four fastest are timed three more times and the best median
   // wins (the first launch of an instance also loads its module).  Cached
   // per class shape and matrix size.
+  uint32_t one = 1u;   // half_kernel.cuh's opaque 1
   struct Cand { int variant, tpb, wpt; double frac; float per; };
   auto time_cand = [&](BatchClass& c, Cand& cd, int reps, float* per_out) -> ld_status {
     BatchClass tc = c;
@@ -454,7 +485,7 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
     for (int rep = 0; rep < reps; ++rep) {
       LD_CUDA(cudaMemsetAsync(args.head, 0, sizeof(unsigned int), b->stream));
       LD_CUDA(cudaEventRecord(b->ev0, b->stream));
-      void* params[] = {&args};
+      void* params[] = {&args, &one};
       LD_CUDA(cudaLaunchKernel(tc.fn(), dim3(class_grid(tc)), dim3(tc.tpb), params, tc.shm(), b->stream));
       LD_CUDA(cudaEventRecord(b->ev1, b->stream));
       LD_CUDA(cudaEventSynchronize(b->ev1));
@@ -491,7 +522,7 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
     double mean = 0;
     for (int p : c.probs) mean += (double)walks[p];
     mean /= std::max<size_t>(1, c.probs.size());
-    const auto key = std::make_tuple(c.D, c.WB, c.WA, (int)std::log2(std::max(1.0, mean)),
+    const auto key = std::make_tuple(c.D, c.WB, c.HW > 0 ? -1 : c.WA, (int)std::log2(std::max(1.0, mean)),
                                      (int)o.batch_split * 1000 + (int)o.threads_per_block * 10 +
                                          (o.batch_row_search > 0 ? 1 : 0));
     {
@@ -568,7 +599,7 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
     if (e != cudaSuccess) break;
     e = cudaStreamWaitEvent(c.stream, b->fork, 0);
     ld::BatchArgs args = class_args(c);
-    void* params[] = {&args};
+    void* params[] = {&args, &one};   // the second one is the two-columns-per-word kernels'
     if (e == cudaSuccess && c.nchunks > 0)
       e = cudaLaunchKernel(c.fn(), dim3(class_grid(c)), dim3(c.tpb), params, c.shm(), c.stream);
     if (e == cudaSuccess) e = cudaEventRecord(c.done, c.stream);
@@ -604,8 +635,8 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
            b->hchunks.size(), (int)std::count_if(b->plans.begin(), b->plans.end(), [](ld_plan* q) { return q != nullptr; }));
   b->desc = buf;
   for (auto& c : b->classes) {
-    snprintf(buf, sizeof buf, "; D=%d int32=%d int8x4=%d: %zu matrices, %d chunks, wpt=%d, tpb=%d, k-%d, grid=%d%s",
-             c.D, c.WB, c.WA, c.probs.size(), c.nchunks, c.wpt, c.tpb, c.kshift, class_grid(c),
+    snprintf(buf, sizeof buf, "; D=%d int32=%d int16x2=%d int8x4=%d: %zu matrices, %d chunks, wpt=%d, tpb=%d, k-%d, grid=%d%s",
+             c.D, c.HW > 0 ? 0 : c.WB, c.HW, c.WA, c.probs.size(), c.nchunks, c.wpt, c.tpb, c.kshift, class_grid(c),
              c.split ? ", column split" : "");
     b->desc += buf;
     if (c.tuned[0] > 0.f && c.tuned[1] > 0.f) {

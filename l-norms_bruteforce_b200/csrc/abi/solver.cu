@@ -22,6 +22,7 @@
 
 #include "smem_limit.h"
 #include "solver_internal.h"
+#include "../kernels/half_kernel.cuh"
 #include "../kernels/registry.h"
 #include "../kernels/split_kernel.cuh"
 #include "../kernels/table_kernel.cuh"
@@ -203,6 +204,91 @@ static bool split_choose(const int64_t* a, int R, int C, int d, int marginal, co
   return found;
 }
 
+// Whether some low-row count lets every column live in 8-bit lanes (the test
+// of table_config), in one pass over the matrix for the column sums and one
+// row more per low-row count.
+static bool narrow_for_some_k(const int64_t* a, int R, int C, int d, int marginal) {
+  std::vector<long long> sum(C, 0), low(C, 0);
+  for (int i = 0; i < R; ++i)
+    for (int l = 0; l < C; ++l) sum[l] += std::llabs(a[(size_t)i * C + l]);
+  if (d >= 2) return *std::max_element(sum.begin(), sum.end()) <= 127;
+  for (int k = 0; k < R && k <= 10; ++k) {
+    bool narrow = true;
+    for (int l = 0; l < C && narrow; ++l) {
+      const long long hb = sum[l] - low[l], lb = low[l];
+      narrow = (marginal && l == 0) ? (2 * hb <= 127 && 2 * lb <= 128) : (hb <= 127 && lb <= 127);
+    }
+    if (narrow) return true;
+    for (int l = 0; l < C; ++l) low[l] += std::llabs(a[(size_t)k * C + l]);
+  }
+  return false;
+}
+
+// Words per lane of the two-columns-per-word form for C columns over S lanes
+// (the instances' steps: 2 words unsplit, 4 split); 0 = no instance.
+static int half_words(int d, int C, int S) {
+  const int step = S == 1 ? 2 : 4, per = 2 * S * step;
+  const int W = (C + per - 1) / per * step;
+  return ld::half_kernel_ptr(d, W, S, 1) ? W : 0;
+}
+
+// The forms with 16-bit values (packed maxima, two columns per word) are
+// allowed, and no other lane width is asked for.
+static bool half_allowed(int d, const ld_options& o) { return d <= 3 && o.lane_bits == 0 && o.pack16 >= 0; }
+
+// Column-split choice of the two-columns-per-word form, for matrices the
+// unsplit kernels do not take (or a forced group size).  Time of a solve:
+// entries x clocks per entry and lane (2.5 per word and message vector, 10 for
+// the seed, the dot product, the ring and the maximum) over the lanes of the
+// GPU, divided by how full they are: four resident blocks keep an SM's four
+// issue slots busy.  Registers decide the resident blocks (half_min_blocks'
+// rule), or the shared memory of the S regions.
+static bool half_split_choose(const int64_t* a, int R, int C, int d, int marginal, const ld_options& o, int sms,
+                              Choice* ch) {
+  const int base = d <= 2 ? 2 : d, F = R - 1;
+  struct Cand { double t; int S, W, k; };
+  std::vector<Cand> cands;
+  for (int S : {2, 4, 8}) {
+    if (o.column_split > 0 && S != o.column_split) continue;
+    const int W = half_words(d, C, S);
+    if (W == 0) continue;
+    const int K = ld::half_kernel_ptr(d, W, S, 2) ? 2 : 1;
+    const int by_regs = ld::half_min_blocks(d, W, S, K);
+    for (int k = 0; k <= F; ++k) {
+      const unsigned long long B = ipow(base, k);
+      if (B > 1024) break;
+      if (o.low_rows >= 0 && k != std::min(o.low_rows, F)) continue;
+      const int Bp = (int)((B + S - 1) / S * S);
+      const size_t smem = (size_t)S * (ld::half_region_words(d, W, R, Bp) + 28) * sizeof(uint32_t);
+      if (smem > 227u * 1024u) break;
+      double units = (double)ipow(base, F - k);
+      if (d >= 3 && !o.enumerate_all && F - k > 0) {
+        uint64_t pass = 0;
+        if (ld_symmetry_walks(d, F - k, 0, ipow(base, F - k), &pass) == LD_OK && pass > 0) units = (double)pass;
+      }
+      const double bps = std::min<double>(by_regs, (double)(228 * 1024 / (smem + 1024)));
+      const double groups = (double)sms * bps * (ld::kTableThreads / S);
+      const double entry = 2.5 * d * W + 10.0, step = 6.0 * d * W + 60.0;
+      const double t = units * ((double)Bp * entry + step) * S / (128.0 * sms) / std::min(1.0, bps / 4.0) /
+                       std::min(1.0, units / groups);
+      cands.push_back({t, S, W, k});
+    }
+  }
+  // the fastest estimate whose layout fits (the layout's bounds take a pass
+  // over the matrix, so only the candidates tried pay for one)
+  std::stable_sort(cands.begin(), cands.end(), [](const Cand& x, const Cand& y) { return x.t < y.t; });
+  for (const Cand& x : cands) {
+    Choice c;
+    if (!half_layout(a, R, C, d, marginal, x.k, x.W, x.S, &c.half)) continue;
+    c.kind = LD_KERNEL_TABLE;
+    c.D = d; c.k = x.k; c.S = x.S; c.HW = x.W;
+    c.lane_bits = 32;
+    *ch = c;
+    return true;
+  }
+  return false;
+}
+
 // Pick the kernel and, for the table kernel, the low-row count minimizing
 // an estimate of the solve time: labelings x (words per labeling + the
 // amortized cost of a high-row step) / threads that have work.
@@ -241,11 +327,27 @@ ld_status choose_kernel(const int64_t* a, int R, int C, int d, int marginal, con
         uint64_t pass = 0;
         if (ld_symmetry_walks(d, F - k, 0, ipow(base, F - k), &pass) == LD_OK && pass > 0) units = (double)pass;
       }
-      const double t = units * (double)B * per_lab / std::min(units, (double)full_threads);
+      double t = units * (double)B * per_lab / std::min(units, (double)full_threads);
       if (!found || t < best_t * 0.999) { best_t = t; *ch = c; found = true; }
+      // two columns per word: a word costs 1.1 absolute-difference-accumulates
+      // (2.5 against 2.27 clocks, 24 words, paired walks), where those cover
+      // one 32-bit or four 8-bit columns
+      const int W = half_allowed(d, o) ? half_words(d, C, 1) : 0;
+      if (W > 0 && 1.1 * W < c.WB + c.WA) {
+        const double hw = 1.1 * d * W + 1.0;
+        t = units * (double)B * (hw + (2.0 * hw + 40.0) / (double)B) / std::min(units, (double)full_threads);
+        if (t < best_t * 0.999 && half_layout(a, R, C, d, marginal, k, W, 1, &c.half)) {
+          best_t = t;
+          c.HW = W;
+          *ch = c;
+        }
+      }
     }
     if (found) return LD_OK;
-    // too wide for one thread's registers: S lanes share each high index
+    // too wide for one thread's registers: S lanes share each high index, in
+    // 8-bit lanes when all columns fit, else two columns per word, else 32-bit
+    if (o.column_split >= 0 && half_allowed(d, o) && !narrow_for_some_k(a, R, C, d, marginal) &&
+        half_split_choose(a, R, C, d, marginal, o, sms, ch)) return LD_OK;
     if (o.column_split >= 0 && split_choose(a, R, C, d, marginal, o, sms, ch)) return LD_OK;
     if (o.column_split > 0)
       return ld_fail(LD_ERR_ARG, "no column-split instance with %d lanes takes d=%d, %d columns", o.column_split, d, C);
@@ -430,7 +532,14 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
     p->k = k;
     p->B = (int)ipow(base, k);
     p->tpb = ld::kTableThreads;
-    if (p->ch.S > 0) {
+    const int HW = p->ch.HW;
+    if (HW > 0) {
+      p->kfn = ld::half_kernel_ptr(D, HW, S, 1);
+      p->Bp = (p->B + S - 1) / S * S;
+      const int region = ld::half_region_words(D, HW, R, p->Bp);
+      p->span = region + (S > 1 ? split_bank_pad(S, ld::half_entry_words(D, HW), region) : 0);
+      p->smem = (size_t)S * p->span * sizeof(uint32_t);
+    } else if (p->ch.S > 0) {
       p->kfn = ld::table_split_kernel_ptr(D, p->ch.PK, p->ch.PW, p->ch.S);
       if (!p->kfn) { delete p; return ld_fail(LD_ERR_ARG, "no column-split kernel for D=%d PW=%d S=%d", D, p->ch.PW, S); }
       p->Bp = (p->B + S - 1) / S * S;
@@ -500,12 +609,13 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
     const unsigned long long want = (mine + per_block - 1) / per_block;
     p->blocks = (int)std::min<unsigned long long>((unsigned long long)di.sms * bps, std::max(1ull, want));
     if (o.blocks > 0) p->blocks = o.blocks;
-    // at least two walks per thread: the instance that walks two high
+    // at least two walks per thread (group): the instance that walks two high
     // indices per thread against each table entry read (L_1 / LM, <= 10
-    // words; d = 2, 3, <= 8 words per vector)
-    if (D <= 3 && p->ch.S == 0 && o.paired_walks >= 0 &&
-        mine >= 2ull * (unsigned long long)p->blocks * (unsigned long long)p->tpb) {
-      const void* pk = ld::table_kernel_pair_ptr(D, p->ch.WB, p->ch.WA, p->ch.lin);
+    // words; d = 2, 3, <= 8 words per vector; two columns per word)
+    if (D <= 3 && (p->ch.S == 0 || HW > 0) && o.paired_walks >= 0 &&
+        mine >= 2ull * (unsigned long long)p->blocks * per_block) {
+      const void* pk = HW > 0 ? ld::half_kernel_ptr(D, HW, S, 2)
+                              : ld::table_kernel_pair_ptr(D, p->ch.WB, p->ch.WA, p->ch.lin);
       int pbps = 0;
       if (pk && ld_raise_smem_limit(pk, p->smem) == cudaSuccess &&
           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pbps, pk, p->tpb, p->smem) == cudaSuccess && pbps >= 1) {
@@ -534,12 +644,13 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
     }
     // vectors of up to 64 words sit at the fixed offsets; wider ones (column
     // split) each take a multiple of 256 bytes
-    const size_t vec = std::max<size_t>(256, align256((size_t)WT * 4));
+    const int vw = HW > 0 ? half_vector_words(HW, S) : WT;   // words of one vector
+    const size_t vec = std::max<size_t>(256, align256((size_t)vw * 4));
     p->off_tot = kOffTot;
     p->off_h0 = kOffTot + vec;
     p->off_tb = kOffTot + 2 * vec;
     p->off_A = kOffTot + 3 * vec;
-    p->upload_bytes = p->off_A + (size_t)R * WT * 4;
+    p->upload_bytes = p->off_A + (size_t)R * vw * 4;
     if (p->sym_digits > 0) {   // completion counts for handing out walks by rank
       p->sym_off = align256(p->upload_bytes);
       p->upload_bytes = p->sym_off + ld_sym_table_len(d, p->sym_digits) * sizeof(uint64_t);
@@ -549,11 +660,22 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
       const ld_status sst = ld_sym_table(d, p->sym_digits, (uint64_t*)(image.data() + p->sym_off));
       if (sst != LD_OK) { delete p; return sst; }
     }
-    pack_row(tot.data(), p->ch, (uint32_t*)(image.data() + p->off_tot));
-    pack_row(h0.data(), p->ch, (uint32_t*)(image.data() + p->off_h0));
-    pack_row(tb.data(), p->ch, (uint32_t*)(image.data() + p->off_tb));
-    for (int i = 0; i < R; ++i)
-      pack_row(a + (size_t)i * C, p->ch, (uint32_t*)(image.data() + p->off_A) + (size_t)i * WT);
+    auto words = [&](size_t off) { return (uint32_t*)(image.data() + off); };
+    if (HW > 0) {   // the bias goes into every vector an H or a T starts from
+      const int64_t* beta = p->ch.half.beta.data();
+      half_pack(tot.data(), beta, C, HW, S, words(p->off_tot));
+      half_pack(h0.data(), beta, C, HW, S, words(p->off_h0));
+      half_pack(tb.data(), beta, C, HW, S, words(p->off_tb));
+      for (int g = 0; g < S; ++g)
+        words(p->off_tb)[g * ld::half_row_words(HW) + HW + 1] = p->ch.half.seed[g];
+      for (int i = 0; i < R; ++i)
+        half_pack(a + (size_t)i * C, nullptr, C, HW, S, words(p->off_A) + (size_t)i * vw);
+    } else {
+      pack_row(tot.data(), p->ch, words(p->off_tot));
+      pack_row(h0.data(), p->ch, words(p->off_h0));
+      pack_row(tb.data(), p->ch, words(p->off_tb));
+      for (int i = 0; i < R; ++i) pack_row(a + (size_t)i * C, p->ch, words(p->off_A) + (size_t)i * WT);
+    }
   } else {
     p->kfn = ld::wide_kernel_ptr(p->ch.i64, p->ch.PC, p->ch.multi, 0);
     if (!p->kfn) { delete p; return ld_fail(LD_ERR_ARG, "no wide kernel for PC=%d", p->ch.PC); }
@@ -640,7 +762,7 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
   p->red.slots = (ld::Slot*)(base_ptr + off_slots);
   // the table kernel's warps fetch walks from a counter in the header (zero
   // in the upload image, reset by each launch's last block)
-  p->red.work = (p->ch.kind == LD_KERNEL_TABLE && p->ch.S == 0 && o.walk_fetch >= 0)
+  p->red.work = (p->ch.kind == LD_KERNEL_TABLE && (p->ch.S == 0 || p->ch.HW > 0) && o.walk_fetch >= 0)
                     ? (unsigned long long*)(base_ptr + kOffWork) : nullptr;
   memcpy(p->res->hstage, image.data(), p->upload_bytes);
   cudaError_t ce = cudaMemcpyAsync(p->res->dmem, p->res->hstage, p->upload_bytes, cudaMemcpyHostToDevice,
@@ -673,7 +795,16 @@ ld_status ldsolve::plan_enqueue(ld_plan* p) {
     // entry's accumulator is at most sum |A| plus twice the LM shift)
     args.pack16 = p->pack16;
     args.red = p->red;
-    if (p->ch.S > 0) {
+    if (p->ch.HW > 0) {
+      ld::HalfArgs hargs;
+      hargs.t = args;
+      hargs.Bp = p->Bp;
+      hargs.span = p->span;
+      hargs.value_bias = p->ch.half.value_bias;
+      hargs.one = 1u;
+      void* params[] = {&hargs};
+      LD_CUDA(cudaLaunchKernel(p->kfn, dim3(p->blocks), dim3(p->tpb), params, p->smem, r->stream));
+    } else if (p->ch.S > 0) {
       ld::SplitArgs sargs;
       sargs.t = args;
       sargs.W = p->ch.WT;
@@ -784,10 +915,10 @@ extern "C" ld_status ld_plan_describe(const ld_plan* p, char* buf, size_t cap) {
   if (p->ch.kind == LD_KERNEL_TABLE)
     snprintf(buf, cap,
              "table D=%d int32 words=%d int8x4 words=%d lin=%d pair=%d k=%d B=%d fw=%d walks=%llu run=%llu "
-             "sym=%d blocks=%d tpb=%d smem=%zu split=%d p16=%d fetch=%d",
-             p->ch.D, p->ch.WB, p->ch.WA, p->ch.lin, p->ch.pair, p->k, p->B, p->fw,
+             "sym=%d blocks=%d tpb=%d smem=%zu split=%d p16=%d fetch=%d half=%d",
+             p->ch.D, p->ch.HW > 0 ? 0 : p->ch.WB, p->ch.HW > 0 ? 0 : p->ch.WA, p->ch.lin, p->ch.pair, p->k, p->B, p->fw,
              (unsigned long long)p->walks, (unsigned long long)p->walks_run, p->sym_digits, p->blocks, p->tpb,
-             p->smem, p->ch.S, p->pack16, p->red.work ? 1 : 0);
+             p->smem, p->ch.S, p->pack16, p->red.work ? 1 : 0, p->ch.HW);
   else
     snprintf(buf, cap, "wide PC=%d multi=%d %s blocks=%d tpb=%d sym=%d walk_len=%llu run=%llu", p->ch.PC,
              p->ch.multi, p->ch.i64 ? "int64" : "int32", p->blocks, p->tpb, p->sym_digits,

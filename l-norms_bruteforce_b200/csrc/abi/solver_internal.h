@@ -11,6 +11,7 @@
 
 #include "../host/ld_internal.h"
 #include "../kernels/common.cuh"
+#include "half_layout.h"
 
 #define LD_CUDA(call)                                                                   \
   do {                                                                                  \
@@ -44,6 +45,9 @@ struct Choice {
   int pair = 0;                               // table: two high indices per thread
   int S = 0, PW = 0, PK = 0;                  // column-split table kernel: lanes per high
                                               // index, words per lane, columns per word
+  int HW = 0;                                 // two columns per word (half_kernel.cuh): words per
+                                              // lane, 0 = the other table kernels
+  HalfLayout half;                            // its biases and seeds
 };
 
 inline int round4(int x) { return (x + 3) & ~3; }

@@ -65,6 +65,21 @@ void split_register_d3(SplitKernelTab& t);
 void split_register_d4_6(SplitKernelTab& t);
 void split_register_d7_10(SplitKernelTab& t);
 const void* table_split_kernel_ptr(int D, int PK, int PW, int S);
+// half_kernel<D, W, S, K> (half_kernel.cuh: two columns per word), D = 1..3, W
+// words per lane, S lanes per high index, K high indices per thread; nullptr
+// when not instantiated.  Instances: S = 1 with W = 2, 4, .., 32 (K = 2: d = 3
+// up to 10 words); S = 2, 4 with W = 4, 8, .., 32 and S = 8 with W = 4 .. 16
+// (d = 3: W up to 16).
+using HalfKernelTab = const void* [4][33][4][2];   // [D][W][log2 S][K - 1]
+void half_register_d1(HalfKernelTab& t);
+void half_register_d2(HalfKernelTab& t);
+void half_register_d3(HalfKernelTab& t);
+void half_register_d1_split(HalfKernelTab& t);
+void half_register_d2_split(HalfKernelTab& t);
+void half_register_d3_split(HalfKernelTab& t);
+const void* half_kernel_ptr(int D, int W, int S, int K);
+// batch_half_kernel<D, W> by (D, W): W = 4, 8, .., 32, or null
+const void* batch_half_kernel_ptr(int D, int W);
 // wide_kernel<IT, PC, MULTI>, PC in {1,2,4,...,128}
 // sym = 1: the instance that takes the walks passing the label-symmetry test by rank
 const void* wide_kernel_ptr(int i64, int PC, int multi, int sym);

@@ -76,6 +76,23 @@ const void* table_split_kernel_ptr(int D, int PK, int PW, int S) {
   return tab[D][PK == 4 ? 1 : 0][pi][si];
 }
 
+const void* half_kernel_ptr(int D, int W, int S, int K) {
+  static HalfKernelTab tab = {};
+  static bool init = [] {
+    half_register_d1(tab);
+    half_register_d2(tab);
+    half_register_d3(tab);
+    half_register_d1_split(tab);
+    half_register_d2_split(tab);
+    half_register_d3_split(tab);
+    return true;
+  }();
+  (void)init;
+  const int si = S == 1 ? 0 : S == 2 ? 1 : S == 4 ? 2 : S == 8 ? 3 : -1;
+  if (D < 1 || D > 3 || W < 1 || W > 32 || si < 0 || K < 1 || K > 2) return nullptr;
+  return tab[D][W][si][K - 1];
+}
+
 static const PruneKernelTab& prune_kernels() {
   static PruneKernelTab tab = {};
   static bool init = [] {
