@@ -26,6 +26,7 @@
 #include "../kernels/registry.h"
 #include "../kernels/split_kernel.cuh"
 #include "../kernels/table_kernel.cuh"
+#include "../kernels/tc_kernel.cuh"
 #include "../kernels/wide_kernel.cuh"
 #include "device_guard.h"
 
@@ -289,6 +290,52 @@ static bool half_split_choose(const int64_t* a, int R, int C, int d, int margina
   return false;
 }
 
+// Shared memory of the tensor-core form; beside the kernel's own arrays (19 KB)
+// it must fit a block's 227 KB.
+constexpr size_t kTcSharedLimit = 227 * 1024 - 20 * 1024;
+static size_t tc_shared(const TcLayout& t, int R, int sym_words) {
+  return ld::tc_smem(t.N, t.steps, R - 1, t.labels, t.WH, sym_words).total;
+}
+
+// The tensor-core form (tc_kernel.cuh), when no option asks for a table
+// kernel's shape and it is estimated faster than `words` words per labeling of
+// the table kernels.  Microseconds per SM, fitted to both sides measured on
+// 11-32 rows of 18-37 columns, d = 1..4: a table launch takes 20 and 1.3 times
+// its 2.3 clocks per word and warp (the seeding and ragged ends of solves of
+// this size); a tensor-core launch 27 (the weights are built and 256 walks
+// seeded per SM), then 0.15 + 0.0345 per step and at least 0.55 for each tile
+// of 128 high indices, and about sqrt(3 tiles) tiles of seeding and waiting at
+// the ends of groups.  The lines cross near 45 us: 24 rows of
+// 33 +-1 columns 38 against 36 us, 26 rows 72 against 47.
+static bool tc_choose(const int64_t* a, int R, int C, int d, int marginal, const ld_options& o, int sms,
+                      double words, Choice* ch) {
+  if (d > 4 || o.lane_bits != 0 || o.low_rows >= 0 || o.threads_per_block > 0 || o.blocks > 0 || o.tile > 0 ||
+      o.column_split != 0 || o.paired_walks < 0 || o.pack16 < 0 || o.walk_fetch < 0)
+    return false;
+  const int base = d <= 2 ? 2 : d, F = R - 1, k = tc_low_rows(d, R);
+  double units = (double)ipow(base, F - k);
+  if (d >= 3 && !o.enumerate_all && F - k > 0) {
+    uint64_t pass = 0;
+    if (ld_symmetry_walks(d, F - k, 0, ipow(base, F - k), &pass) == LD_OK && pass > 0) units = (double)pass;
+  }
+  const double per_sm = units / ((double)(o.shard_count > 1 ? o.shard_count : 1) * sms), tiles = per_sm / 128.0;
+  const double table = 20.0 + 1.3 * per_sm * (double)ipow(base, k) * 2.3 * words / (128.0 * 1965.0);
+  auto mine = [&](int steps) {
+    return 27.0 + (tiles + std::sqrt((d >= 3 ? 8.0 : 3.0) * tiles)) * std::max(0.55, 0.15 + 0.0345 * steps);
+  };
+  if (mine(2) > table) return false;
+  TcLayout lay;
+  if (!tc_layout(a, R, C, d, marginal, k, &lay) || mine(lay.steps) > table) return false;
+  // with the completion counts of any walk length
+  const size_t sym_words = d >= 3 && !o.enumerate_all ? ld_sym_table_len(d, F - k) : 0;
+  if (tc_shared(lay, R, (int)sym_words) > kTcSharedLimit) return false;
+  ch->kind = LD_KERNEL_TABLE;
+  ch->D = d; ch->k = k; ch->S = 0; ch->HW = 0; ch->lin = 0;
+  ch->tc = true;
+  ch->tcl = std::move(lay);
+  return true;
+}
+
 // Pick the kernel and, for the table kernel, the low-row count minimizing
 // an estimate of the solve time: labelings x (words per labeling + the
 // amortized cost of a high-row step) / threads that have work.
@@ -343,7 +390,10 @@ ld_status choose_kernel(const int64_t* a, int R, int C, int d, int marginal, con
         }
       }
     }
-    if (found) return LD_OK;
+    if (found) {
+      tc_choose(a, R, C, d, marginal, o, sms, (ch->HW > 0 ? 1.1 * ch->HW : ch->WB + ch->WA) * d, ch);
+      return LD_OK;
+    }
     // too wide for one thread's registers: S lanes share each high index, in
     // 8-bit lanes when all columns fit, else two columns per word, else 32-bit
     if (o.column_split >= 0 && half_allowed(d, o) && !narrow_for_some_k(a, R, C, d, marginal) &&
@@ -533,7 +583,14 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
     p->B = (int)ipow(base, k);
     p->tpb = ld::kTableThreads;
     const int HW = p->ch.HW;
-    if (HW > 0) {
+    const bool tc = p->ch.tc;
+    if (tc) {
+      const TcLayout& t = p->ch.tcl;
+      p->kfn = ld::tc_kernel_ptr(d <= 2 ? 2 : d, t.WH, t.steps);
+      p->tpb = ld::kTcThreads;
+      p->ch.pair = 1;             // many high indices against each table entry
+      p->ch.lin = marginal ? 1 : 0;
+    } else if (HW > 0) {
       p->kfn = ld::half_kernel_ptr(D, HW, S, 1);
       p->Bp = (p->B + S - 1) / S * S;
       const int region = ld::half_region_words(D, HW, R, p->Bp);
@@ -556,6 +613,20 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
       }
       p->smem = (size_t)ld::table_smem_words(D, WT, R, p->B) * sizeof(uint32_t);
     }
+    const int nh = F - k;
+    // d >= 3: walks that hold no smallest index of a label-permutation
+    // class are skipped (symmetry.c); the walks that run decide the length
+    const bool sym = D >= 3 && !o.enumerate_all;
+    auto walks_run = [&](int f, unsigned long long lo, unsigned long long hi) -> unsigned long long {
+      uint64_t c = hi - lo;
+      if (sym && nh - f > 0 && ld_symmetry_walks(d, nh - f, lo, hi, &c) != LD_OK) c = hi - lo;
+      return (unsigned long long)c;
+    };
+    if (tc) {   // one CTA per SM: the weights take most of the shared memory, and the kernel all of TMEM
+      const TcLayout& t = p->ch.tcl;
+      const int digits = sym ? nh : 0;   // room for the completion counts of any walk length
+      p->smem = std::max<size_t>(120 * 1024, tc_shared(t, R, digits > 0 ? (int)ld_sym_table_len(d, digits) : 0));
+    }
     if (ld_raise_smem_limit(p->kfn, p->smem) != cudaSuccess) {
       delete p; return ld_fail(LD_ERR_CUDA, "cannot reserve %zu bytes of shared memory", p->smem);
     }
@@ -566,25 +637,25 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
     // packed maxima: the table kernel's scans (the column split keeps one maximum per word)
     p->pack16 = (p->ch.S == 0 && o.pack16 >= 0 && p->bounds.total + 2 * (marginal ? p->bounds.K : 0) < 65536) ? 1 : 0;
     // parallel units of a full grid: threads, or groups of S lanes
-    const unsigned long long full = (unsigned long long)di.sms * bps * (p->tpb / S);
-    const int nh = F - k;
-    // d >= 3: walks that hold no smallest index of a label-permutation
-    // class are skipped (symmetry.c); the walks that run decide the length
-    const bool sym = D >= 3 && !o.enumerate_all;
-    auto walks_run = [&](int f, unsigned long long lo, unsigned long long hi) -> unsigned long long {
-      uint64_t c = hi - lo;
-      if (sym && nh - f > 0 && ld_symmetry_walks(d, nh - f, lo, hi, &c) != LD_OK) c = hi - lo;
-      return (unsigned long long)c;
-    };
+    const unsigned long long full = (unsigned long long)di.sms * bps * (tc ? 128 : p->tpb / S);
     // walk length: as long as the walks still number >= 16 per thread of a
     // full grid (d <= 2), or >= 4 (d >= 3, whose walk seeding costs 64-bit
     // divisions per high digit).  Longer walks seed less often; the kernel is
     // issue-bound, so warps left with one walk more than others finish
     // faster as the rest drain.  Measured: 20x30 d = 3 9 % faster at 4 than
     // at 32; 34x37 LM 3 % faster at 16 than at 32, 12 % slower at 8.
+    // The tensor-core form takes 128 walks at a time.  Setting up a group of
+    // walks costs about a tile (d >= 3: three), and a CTA waits for half a
+    // group at the end: of n tiles per CTA, walks of sqrt(2 n) (sqrt(6 n))
+    // lose least.
     const unsigned long long per_thread = D >= 3 ? 4ull : 16ull;
     int fw = 0;
-    while (fw < nh && walks_run(fw + 1, 0, ipow(base, nh - fw - 1)) >= per_thread * full) ++fw;
+    if (tc) {
+      const double tiles = (double)walks_run(0, 0, ipow(base, nh)) / ((double)di.sms * 128.0);
+      const double longest = std::min(std::sqrt((D >= 3 ? 6.0 : 2.0) * tiles) * 1.4, (double)(1 << 30));
+      while (fw < nh && (double)ipow(base, fw + 1) <= longest) ++fw;
+    }
+    while (!tc && fw < nh && walks_run(fw + 1, 0, ipow(base, nh - fw - 1)) >= per_thread * full) ++fw;
     if (o.tile > 0) fw = std::min(nh, o.tile);
     p->fw = fw;
     p->walk_len = ipow(base, fw);
@@ -605,14 +676,14 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
       p->rank_end = p->rank_begin + p->walks_run;
     }
     const unsigned long long mine = p->walks_run;
-    const unsigned long long per_block = (unsigned long long)(p->tpb / S);
+    const unsigned long long per_block = tc ? 128ull : (unsigned long long)(p->tpb / S);
     const unsigned long long want = (mine + per_block - 1) / per_block;
     p->blocks = (int)std::min<unsigned long long>((unsigned long long)di.sms * bps, std::max(1ull, want));
     if (o.blocks > 0) p->blocks = o.blocks;
     // at least two walks per thread (group): the instance that walks two high
     // indices per thread against each table entry read (L_1 / LM, <= 10
     // words; d = 2, 3, <= 8 words per vector; two columns per word)
-    if (D <= 3 && (p->ch.S == 0 || HW > 0) && o.paired_walks >= 0 &&
+    if (!tc && D <= 3 && (p->ch.S == 0 || HW > 0) && o.paired_walks >= 0 &&
         mine >= 2ull * (unsigned long long)p->blocks * per_block) {
       const void* pk = HW > 0 ? ld::half_kernel_ptr(D, HW, S, 2)
                               : ld::table_kernel_pair_ptr(D, p->ch.WB, p->ch.WA, p->ch.lin);
@@ -651,6 +722,15 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
     p->off_tb = kOffTot + 2 * vec;
     p->off_A = kOffTot + 3 * vec;
     p->upload_bytes = p->off_A + (size_t)R * vw * 4;
+    const TcLayout& t = p->ch.tcl;
+    const std::vector<uint32_t>* parts[9] = {&t.hinit, &t.tinit, &t.tmin, &t.always, &t.once, &t.delta, &t.prog,
+                                             &t.feat, &t.consts};
+    if (tc) {
+      size_t at = kOffTot;
+      for (int i = 0; i < 9; ++i) { p->off_tc[i] = at; at = (at + parts[i]->size() * 4 + 15) & ~(size_t)15; }
+      p->off_tc[9] = at;
+      p->upload_bytes = at + t.raw.size() * 4;
+    }
     if (p->sym_digits > 0) {   // completion counts for handing out walks by rank
       p->sym_off = align256(p->upload_bytes);
       p->upload_bytes = p->sym_off + ld_sym_table_len(d, p->sym_digits) * sizeof(uint64_t);
@@ -661,7 +741,10 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
       if (sst != LD_OK) { delete p; return sst; }
     }
     auto words = [&](size_t off) { return (uint32_t*)(image.data() + off); };
-    if (HW > 0) {   // the bias goes into every vector an H or a T starts from
+    if (tc) {
+      for (int i = 0; i < 9; ++i) memcpy(words(p->off_tc[i]), parts[i]->data(), parts[i]->size() * 4);
+      memcpy(words(p->off_tc[9]), t.raw.data(), t.raw.size() * 4);
+    } else if (HW > 0) {   // the bias goes into every vector an H or a T starts from
       const int64_t* beta = p->ch.half.beta.data();
       half_pack(tot.data(), beta, C, HW, S, words(p->off_tot));
       half_pack(h0.data(), beta, C, HW, S, words(p->off_h0));
@@ -795,7 +878,30 @@ ld_status ldsolve::plan_enqueue(ld_plan* p) {
     // entry's accumulator is at most sum |A| plus twice the LM shift)
     args.pack16 = p->pack16;
     args.red = p->red;
-    if (p->ch.HW > 0) {
+    if (p->ch.tc) {
+      const TcLayout& t = p->ch.tcl;
+      auto at = [&](int i) { return (const uint32_t*)(base_ptr + p->off_tc[i]); };
+      ld::TcArgs targs;
+      targs.hinit = at(0); targs.tinit = at(1); targs.tmin = at(2); targs.always = at(3); targs.once = at(4);
+      targs.delta = at(5); targs.prog = (const uint4*)at(6); targs.feat = (const uint2*)at(7);
+      targs.consts = at(8); targs.raw = (const int*)at(9);
+      targs.R = p->R; targs.C = p->C; targs.d = p->d; targs.marginal = p->marginal;
+      targs.k = p->k; targs.B = p->B; targs.N = t.N;
+      targs.labels = t.labels;
+      targs.parity = t.parity;
+      targs.nconst = (int)t.consts.size();
+      targs.walk_len = p->walk_len;
+      targs.fw = p->fw;
+      targs.it_begin = p->sym_digits > 0 ? p->rank_begin : p->walk_begin;
+      targs.it_end = p->sym_digits > 0 ? p->rank_end : p->walk_end;
+      targs.sym_digits = p->sym_digits;
+      targs.sym_words = p->sym_digits > 0 ? (int)ld_sym_table_len(p->d, p->sym_digits) : 0;
+      targs.sym_table = args.sym_table;
+      targs.value_offset = p->value_offset;
+      targs.red = p->red;
+      void* params[] = {&targs};
+      LD_CUDA(cudaLaunchKernel(p->kfn, dim3(p->blocks), dim3(p->tpb), params, p->smem, r->stream));
+    } else if (p->ch.HW > 0) {
       ld::HalfArgs hargs;
       hargs.t = args;
       hargs.Bp = p->Bp;
@@ -861,6 +967,8 @@ ld_status ldsolve::plan_fetch(ld_plan* p, ld_result* res, int32_t* strategy) {
   LD_CUDA(cudaStreamSynchronize(r->stream));
   float ms = 0.f;
   LD_CUDA(cudaEventElapsedTime(&ms, r->ev0, r->ev1));
+  if (p->ch.kind == LD_KERNEL_TABLE && p->ch.tc && h->value == LLONG_MAX)
+    return ld_fail(LD_ERR_TIMEOUT, "tensor-core enumeration: a device-side wait ran out");
   memset(res, 0, sizeof *res);
   res->value = h->value;
   res->gray_index = h->index;
@@ -915,10 +1023,11 @@ extern "C" ld_status ld_plan_describe(const ld_plan* p, char* buf, size_t cap) {
   if (p->ch.kind == LD_KERNEL_TABLE)
     snprintf(buf, cap,
              "table D=%d int32 words=%d int8x4 words=%d lin=%d pair=%d k=%d B=%d fw=%d walks=%llu run=%llu "
-             "sym=%d blocks=%d tpb=%d smem=%zu split=%d p16=%d fetch=%d half=%d",
+             "sym=%d blocks=%d tpb=%d smem=%zu split=%d p16=%d fetch=%d half=%d tc=%d",
              p->ch.D, p->ch.HW > 0 ? 0 : p->ch.WB, p->ch.HW > 0 ? 0 : p->ch.WA, p->ch.lin, p->ch.pair, p->k, p->B, p->fw,
              (unsigned long long)p->walks, (unsigned long long)p->walks_run, p->sym_digits, p->blocks, p->tpb,
-             p->smem, p->ch.S, p->pack16, p->red.work ? 1 : 0, p->ch.HW);
+             p->smem, p->ch.S, p->pack16, p->red.work ? 1 : 0, p->ch.HW,
+             p->ch.tc ? 16 * p->ch.tcl.steps : 0);
   else
     snprintf(buf, cap, "wide PC=%d multi=%d %s blocks=%d tpb=%d sym=%d walk_len=%llu run=%llu", p->ch.PC,
              p->ch.multi, p->ch.i64 ? "int64" : "int32", p->blocks, p->tpb, p->sym_digits,

@@ -12,6 +12,7 @@
 #include "../host/ld_internal.h"
 #include "../kernels/common.cuh"
 #include "half_layout.h"
+#include "tc_layout.h"
 
 #define LD_CUDA(call)                                                                   \
   do {                                                                                  \
@@ -48,6 +49,8 @@ struct Choice {
   int HW = 0;                                 // two columns per word (half_kernel.cuh): words per
                                               // lane, 0 = the other table kernels
   HalfLayout half;                            // its biases and seeds
+  bool tc = false;                            // tensor-core enumeration (tc_kernel.cuh)
+  TcLayout tcl;                               // its images
 };
 
 inline int round4(int x) { return (x + 3) & ~3; }
@@ -129,6 +132,7 @@ struct ld_plan {
   size_t off_tot = 0, off_h0 = 0, off_tb = 0, off_A = 0;
   int Bp = 0, span = 0;                           // column split: table entries, words per slice region
   int pack16 = 0;                                 // table kernel: packed 16-bit maxima
+  size_t off_tc[10] = {};                          // tensor-core form: image offsets (TcArgs' order)
   bool uploaded = false;       // the upload belongs to the next fetched launch
   ld::Reduce red{};
   const void* kfn = nullptr;

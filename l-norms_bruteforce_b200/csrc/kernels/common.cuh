@@ -74,8 +74,9 @@ __device__ __forceinline__ void warp_best(long long& v, unsigned long long& n) {
 // Block-wide best, then one atomicMax per block on the value and a slot
 // write; the last block to finish picks the smallest index among the slots
 // that reach the maximum and re-arms the scratch for the next launch.
-// Must be called by every thread of the block.
-__device__ __forceinline__ void grid_reduce(long long v, unsigned long long n, const Reduce& R) {
+// Must be called by every thread of the block; true in the last block to
+// finish (which has written the result).
+__device__ __forceinline__ bool grid_reduce(long long v, unsigned long long n, const Reduce& R) {
   __shared__ long long s_v[32];
   __shared__ unsigned long long s_n[32];
   __shared__ bool s_last;
@@ -98,7 +99,7 @@ __device__ __forceinline__ void grid_reduce(long long v, unsigned long long n, c
     }
   }
   __syncthreads();
-  if (!s_last) return;
+  if (!s_last) return false;
   __threadfence();
   const long long gmax = *((volatile long long*)R.gvalue);
   unsigned long long bn = ULLONG_MAX;
@@ -122,6 +123,7 @@ __device__ __forceinline__ void grid_reduce(long long v, unsigned long long n, c
     if (R.work) *R.work = 0ull;   // every block has finished fetching walks
     __threadfence();
   }
+  return true;
 }
 
 }  // namespace ld

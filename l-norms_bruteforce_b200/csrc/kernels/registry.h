@@ -80,6 +80,13 @@ void half_register_d3_split(HalfKernelTab& t);
 const void* half_kernel_ptr(int D, int W, int S, int K);
 // batch_half_kernel<D, W> by (D, W): W = 4, 8, .., 32, or null
 const void* batch_half_kernel_ptr(int D, int W);
+// tc_kernel<D, WH, S> (tc_kernel.cuh, tensor cores): D = 2 (d = 1, 2), 3, 4,
+// WH = 1..8, S = 2, 4, .., 30, WH <= S <= 12 WH; nullptr when not instantiated
+using TcKernelTab = const void* [3][8][15];
+void tc_register_d2(TcKernelTab& t);
+void tc_register_d3(TcKernelTab& t);
+void tc_register_d4(TcKernelTab& t);
+const void* tc_kernel_ptr(int D, int WH, int S);
 // wide_kernel<IT, PC, MULTI>, PC in {1,2,4,...,128}
 // sym = 1: the instance that takes the walks passing the label-symmetry test by rank
 const void* wide_kernel_ptr(int i64, int PC, int multi, int sym);

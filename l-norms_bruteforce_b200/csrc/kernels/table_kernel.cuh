@@ -486,8 +486,8 @@ __device__ __forceinline__ bool walk_holds_class_min(unsigned long long wk, int 
 // digit DP of symmetry.c, which holds the host copy of this function).  Digit
 // by digit from the top, the digit is the first whose passing continuations
 // reach past i; once at most one label is unseen every continuation passes
-// and the rest of i is the remaining digits.
-template <int D>
+// and the rest of i is the remaining digits.  GLOBAL: f is in global memory.
+template <int D, bool GLOBAL = true>
 __device__ __forceinline__ unsigned long long walk_of_rank(unsigned long long i, int P,
                                                            const unsigned long long* __restrict__ f) {
   unsigned used = 1u;
@@ -501,7 +501,8 @@ __device__ __forceinline__ unsigned long long walk_of_rank(unsigned long long i,
       lab = par ? D - 1 - n : n;
       if (!(((used >> lab) & 1u) || lab == want)) continue;
       np = (D & 1) ? (par ^ (n & 1)) : (n & 1);
-      const unsigned long long c = __ldg(f + ((size_t)((used | (1u << lab)) >> 1) * 2 + np) * (size_t)(P + 1) + q);
+      const unsigned long long* at = f + ((size_t)((used | (1u << lab)) >> 1) * 2 + np) * (size_t)(P + 1) + q;
+      const unsigned long long c = GLOBAL ? __ldg(at) : *at;
       if (i < c) break;
       i -= c;
     }

@@ -1,0 +1,6 @@
+// tc_kernel<2, WH, S> (d = 1 and 2): WH = 1..8 H words, S = 2, 4, .., 30 steps
+// (at least one and at most twelve per word).
+#include "tc_inst.cuh"
+namespace ld {
+void tc_register_d2(TcKernelTab& t) { inst::fill_tc<2>(t, std::make_integer_sequence<int, kTcMaxWords * kTcMaxSteps / 2>{}); }
+}  // namespace ld

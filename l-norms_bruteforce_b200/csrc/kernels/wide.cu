@@ -93,6 +93,19 @@ const void* half_kernel_ptr(int D, int W, int S, int K) {
   return tab[D][W][si][K - 1];
 }
 
+const void* tc_kernel_ptr(int D, int WH, int S) {
+  static TcKernelTab tab = {};
+  static bool init = [] {
+    tc_register_d2(tab);
+    tc_register_d3(tab);
+    tc_register_d4(tab);
+    return true;
+  }();
+  (void)init;
+  if (D < 2 || D > 4 || WH < 1 || WH > 8 || S < 2 || S > 30 || S % 2) return nullptr;
+  return tab[D - 2][WH - 1][S / 2 - 1];
+}
+
 static const PruneKernelTab& prune_kernels() {
   static PruneKernelTab tab = {};
   static bool init = [] {

@@ -1,0 +1,99 @@
+"""The tensor-core enumeration (tc_kernel.cuh), which large solves of matrices
+with small entries take: bit-exact against the oracle (value and smallest
+Gray index) for d = 1, LM, 2, 3 and 4, over column counts at the edges of the
+byte words, +-1 entries (ties, both parities of a column's sum), entries to
++-3, one-sided columns, equal rows, zero columns, shards, label symmetry on
+and off, repeated launches of a plan, and inside a batch."""
+import numpy as np
+import pytest
+
+import oracle_ffi as O
+
+pytestmark = pytest.mark.gpu
+
+ROWS = {1: 27, 2: 27, 3: 17, 4: 14}
+
+
+def _solve(ld, a, d, marg, **kw):
+    plan = ld.Plan(a, d, marg, ld.options(**kw))
+    desc = plan.describe()
+    sol = plan.solve()
+    plan.close()
+    return sol, desc
+
+
+def _tc(desc):
+    return int(desc.split("tc=")[1].split()[0])
+
+
+def _matrix(rng, d, cols, kind, rows=0):
+    shape = (rows or ROWS[d], cols)
+    if kind == "pm1":
+        return rng.choice(np.array([-1, 1], dtype=np.int64), size=shape)
+    if kind == "sparse":
+        a = rng.integers(-1, 2, size=shape)
+        a[:, cols // 2] = 0
+        a[2] = a[1]
+        return a.astype(np.int64)
+    a = rng.integers(-3, 4, size=shape).astype(np.int64)
+    a[:, -1] = np.abs(a[:, -1])
+    return a
+
+
+@pytest.mark.parametrize("kind", ["pm1", "sparse", "amp3"])
+@pytest.mark.parametrize("d,marg,cols", [(1, False, 9), (1, False, 16), (1, False, 33), (1, True, 37), (1, True, 48),
+                                         (2, False, 11), (2, False, 16), (2, False, 24), (3, False, 10),
+                                         (3, False, 17), (3, False, 30), (4, False, 8), (4, False, 21)])
+def test_matches_the_oracle(ld, d, marg, cols, kind):
+    rng = np.random.default_rng(100 * d + cols + len(kind))
+    a = _matrix(rng, d, cols, kind)
+    if marg:
+        a[:, 0] = rng.integers(-5, 6, size=a.shape[0])
+    ref = O.enumerate_max(a, d, marg)
+    sol, desc = _solve(ld, a, d, marg)
+    assert _tc(desc) > 0 or kind == "amp3" or cols < 12, desc
+    assert (sol.value, sol.gray_index) == ref, desc
+    table, desc = _solve(ld, a, d, marg, paired_walks=-1)
+    assert _tc(desc) == 0 and (table.value, table.gray_index) == ref, desc
+    assert sol.evaluated <= sol.labelings == table.labelings
+
+
+@pytest.mark.parametrize("d,rows,cols", [(1, 28, 36), (3, 18, 28)])
+def test_shards_launches_and_every_walk(ld, d, rows, cols):
+    rng = np.random.default_rng(rows)
+    a = _matrix(rng, d, cols, "pm1", rows)
+    ref = O.enumerate_max(a, d, False)
+    plan = ld.Plan(a, d)
+    assert _tc(plan.describe()) > 0, plan.describe()
+    whole = plan.solve()
+    for _ in range(3):
+        again = plan.solve()
+        assert (again.value, again.gray_index) == (whole.value, whole.gray_index) == ref
+    plan.close()
+    best, lo, work = None, 0, 0
+    for i in range(2):
+        plan = ld.Plan(a, d, False, ld.options(shard_index=i, shard_count=2))
+        assert plan.range[0] == lo
+        lo = plan.range[1]
+        sol = plan.solve()
+        plan.close()
+        cand = (sol.value, -sol.gray_index)
+        best = cand if best is None or cand > best else best
+        work += sol.evaluated
+    assert lo == O.total(rows, d) and (best[0], -best[1]) == ref
+    if d >= 3:
+        full, desc = _solve(ld, a, d, False, enumerate_all=1)
+        assert _tc(desc) > 0 and (full.value, full.gray_index) == ref
+        assert whole.evaluated < full.evaluated == full.labelings
+
+
+def test_a_block_of_ties(ld):
+    """Every labeling of the low rows ties: the smallest index is reported."""
+    a = np.zeros((28, 40), dtype=np.int64)
+    a[:, :20] = 1
+    a[12:, 20:] = np.random.default_rng(3).choice([-1, 1], size=(16, 20))
+    a[:12, :20] = 0
+    a[:12, 20] = 1
+    ref = O.enumerate_max(a, 1, False)
+    sol, desc = _solve(ld, a, 1, False)
+    assert (sol.value, sol.gray_index) == ref, desc
