@@ -57,44 +57,60 @@ Bounds compute_bounds(const int64_t* a, int R, int C, int marginal) {
 
 
 
+// Whether a column's lanes can be 8 bits wide, given the absolute sums of its
+// high (with the fixed row) and low rows.  For d = 1 the two operands of each
+// absolute difference are the high rows' partial sum and the low rows', so
+// each only needs its own part to fit 8 bits; for LM, column 0 carries the
+// shift K split the same way (K_H + K_L).  For d >= 2 a table vector holds the
+// column total minus low rows, so a column is narrow when its full bound fits.
+static bool narrow_column(long long hb, long long lb, int d, int marginal, int l, int force_bits) {
+  if (force_bits == 32) return false;
+  if (d == 1) return (marginal && l == 0) ? (2 * hb <= 127 && 2 * lb <= 128) : (hb <= 127 && lb <= 127);
+  return hb + lb <= 127;
+}
+
+// The instance for `wide` 32-bit and `narrow` 8-bit columns: its int32 and
+// int8x4 words (all columns wide when there is no mixed instance).  Returns
+// false if none exists.
+static bool instance_words(int wide, int narrow, int d, int force_bits, int* WB, int* WA) {
+  const int C = wide + narrow;
+  if (force_bits == 8 && wide > 0) return false;
+  *WB = wide;
+  *WA = (narrow + 3) / 4;
+  if (d >= 2 && *WB > 0 && *WA > 0) { *WB = C; *WA = 0; }   // no mixed instances for d >= 2
+  if (d >= 4 && *WA == 0) *WB = round4(*WB);   // d >= 4: 32-bit instances come in multiples of 4 words
+  if (!ld::table_kernel_mixed_ptr(d, *WB, *WA)) {
+    if (force_bits == 8 || C > 64 || !ld::table_kernel_mixed_ptr(d, C, 0)) return false;
+    *WB = C;
+    *WA = 0;
+  }
+  return true;
+}
+
+// The words of table_config from the columns' absolute sums and their low rows' part.
+static bool table_words(const long long* sum, const long long* low, int C, int d, int marginal, int force_bits,
+                        int* WB, int* WA) {
+  int narrow = 0;
+  for (int l = 0; l < C; ++l) narrow += narrow_column(sum[l] - low[l], low[l], d, marginal, l, force_bits);
+  return instance_words(C - narrow, narrow, d, force_bits, WB, WA);
+}
+
 // Table-kernel configuration for a given number of low rows k: which columns
-// can live in 8-bit lanes.  For d = 1 the two operands of each absolute
-// difference are the high rows' partial sum (with the fixed row) and the low
-// rows' partial sum, so each only needs its own part to fit 8 bits; for LM,
-// column 0 carries the shift K split the same way (K_H + K_L).  For d >= 2 a
-// table vector holds the column total minus low rows, so a column is narrow
-// when its full bound fits.  Returns false if no instance exists.
+// live in 8-bit lanes (they follow the others).  Returns false if no instance
+// exists.
 bool table_config(const int64_t* a, int R, int C, int d, int marginal, int k, int force_bits,
                   Choice* ch) {
+  std::vector<long long> hb(C, 0), lb(C, 0);
+  for (int i = 0; i < R; ++i)
+    for (int l = 0; l < C; ++l) (i < k ? lb : hb)[l] += std::llabs(a[(size_t)i * C + l]);
   std::vector<int> wide, narrow;
-  for (int l = 0; l < C; ++l) {
-    long long hb = 0, lb = 0;
-    for (int i = 0; i < R; ++i) {
-      const int64_t v = a[(size_t)i * C + l];
-      const long long av = v < 0 ? -(long long)v : (long long)v;
-      if (i < k) lb += av; else hb += av;
-    }
-    bool nar;
-    if (d == 1) nar = (marginal && l == 0) ? (2 * hb <= 127 && 2 * lb <= 128) : (hb <= 127 && lb <= 127);
-    else nar = hb + lb <= 127;
-    if (force_bits == 32) nar = false;
-    (nar ? narrow : wide).push_back(l);
-  }
-  if (force_bits == 8 && !wide.empty()) return false;
-  int WB = (int)wide.size(), WA = ((int)narrow.size() + 3) / 4;
-  if (d >= 2 && WB > 0 && WA > 0) {             // no mixed instances for d >= 2
-    if (force_bits == 8) return false;
-    wide.insert(wide.end(), narrow.begin(), narrow.end());
+  for (int l = 0; l < C; ++l) (narrow_column(hb[l], lb[l], d, marginal, l, force_bits) ? narrow : wide).push_back(l);
+  int WB = 0, WA = 0;
+  if (!instance_words((int)wide.size(), (int)narrow.size(), d, force_bits, &WB, &WA)) return false;
+  if (WA == 0 && !narrow.empty()) {             // every column in 32-bit lanes
+    if (d >= 2 && !wide.empty()) wide.insert(wide.end(), narrow.begin(), narrow.end());
+    else { wide.resize(C); for (int l = 0; l < C; ++l) wide[l] = l; }
     narrow.clear();
-    WB = C; WA = 0;
-  }
-  if (d >= 4 && WA == 0) WB = round4(WB);      // d >= 4: 32-bit instances come in multiples of 4 words
-  if (!ld::table_kernel_mixed_ptr(d, WB, WA)) {
-    if (force_bits == 8 || C > 64 || !ld::table_kernel_mixed_ptr(d, C, 0)) return false;
-    wide.clear();
-    for (int l = 0; l < C; ++l) wide.push_back(l);
-    narrow.clear();
-    WB = C; WA = 0;
   }
   ch->kind = LD_KERNEL_TABLE;
   ch->D = d; ch->WB = WB; ch->WA = WA; ch->WT = round4(WB + WA); ch->k = k;
@@ -107,15 +123,17 @@ bool table_config(const int64_t* a, int R, int C, int d, int marginal, int k, in
 // Bank padding of the column-split kernel's slice regions: the S lanes of a
 // group read, at step r of a tile, entry (g + r) mod S of slice g; with
 // 16-byte loads a quarter warp is served in one pass when those S addresses
-// fall on distinct groups of four banks.  Returns the padding (a multiple of
-// 4 words, below 32) with the fewest repeated bank groups over all r.
+// fall on distinct groups of four banks.  Seeds and steps read the same row of
+// every slice, a distance of the span alone.  Returns the padding (a multiple
+// of 4 words, below 32) with the fewest repeated bank groups over all r and
+// the row (without the row a 24 x 128 d = 1 solve of four lanes took 158 us).
 int split_bank_pad(int S, int NW, int span) {
   int best_pad = 0, best_cost = INT_MAX;
   for (int pad = 0; pad < 32; pad += 4) {
     int cost = 0;
-    for (int r = 0; r < S; ++r) {
+    for (int r = 0; r <= S; ++r) {   // r = S: the row
       int cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      for (int g = 0; g < S; ++g) cnt[((g * (span + pad) + ((g + r) % S) * NW) / 4) & 7]++;
+      for (int g = 0; g < S; ++g) cnt[((g * (span + pad) + (r < S ? (g + r) % S : 0) * NW) / 4) & 7]++;
       for (int c : cnt) cost += c > 1 ? c - 1 : 0;
     }
     if (cost < best_cost) { best_cost = cost; best_pad = pad; }
@@ -238,12 +256,15 @@ static int half_words(int d, int C, int S) {
 static bool half_allowed(int d, const ld_options& o) { return d <= 3 && o.lane_bits == 0 && o.pack16 >= 0; }
 
 // Column-split choice of the two-columns-per-word form, for matrices the
-// unsplit kernels do not take (or a forced group size).  Time of a solve:
-// entries x clocks per entry and lane (2.5 per word and message vector, 10 for
-// the seed, the dot product, the ring and the maximum) over the lanes of the
-// GPU, divided by how full they are: four resident blocks keep an SM's four
-// issue slots busy.  Registers decide the resident blocks (half_min_blocks'
-// rule), or the shared memory of the S regions.
+// unsplit kernels do not take (or a forced group size).  A group takes its
+// high indices in rounds, two at once when every group has two: clocks per
+// entry and lane are 2.5 per word and message vector (3.8 one at a time: each
+// read serves half the work, measured 1.5x) and 10 for the seed word, the dot
+// product, the ring and the maximum; resident warps share the issue slots,
+// and fewer than three blocks do not fill them.  Registers decide the resident
+// blocks (half_min_blocks), or the shared memory of the S regions.  Measured
+// against the other group sizes: 28 x 256, d = 1, four lanes 1.30 ms, eight
+// 1.47; 24 x 128 two lanes 0.090, four 0.096, eight 0.100.
 static bool half_split_choose(const int64_t* a, int R, int C, int d, int marginal, const ld_options& o, int sms,
                               Choice* ch) {
   const int base = d <= 2 ? 2 : d, F = R - 1;
@@ -253,8 +274,8 @@ static bool half_split_choose(const int64_t* a, int R, int C, int d, int margina
     if (o.column_split > 0 && S != o.column_split) continue;
     const int W = half_words(d, C, S);
     if (W == 0) continue;
-    const int K = ld::half_kernel_ptr(d, W, S, 2) ? 2 : 1;
-    const int by_regs = ld::half_min_blocks(d, W, S, K);
+    const bool paired = ld::half_kernel_ptr(d, W, S, 2) != nullptr && o.paired_walks >= 0;
+    const int by_regs = ld::half_min_blocks(d, W, S, paired ? 2 : 1);
     for (int k = 0; k <= F; ++k) {
       const unsigned long long B = ipow(base, k);
       if (B > 1024) break;
@@ -267,11 +288,15 @@ static bool half_split_choose(const int64_t* a, int R, int C, int d, int margina
         uint64_t pass = 0;
         if (ld_symmetry_walks(d, F - k, 0, ipow(base, F - k), &pass) == LD_OK && pass > 0) units = (double)pass;
       }
-      const double bps = std::min<double>(by_regs, (double)(228 * 1024 / (smem + 1024)));
+      const double bps = std::max(1.0, std::min<double>(by_regs, (double)(228 * 1024 / (smem + 1024))));
       const double groups = (double)sms * bps * (ld::kTableThreads / S);
-      const double entry = 2.5 * d * W + 10.0, step = 6.0 * d * W + 60.0;
-      const double t = units * ((double)Bp * entry + step) * S / (128.0 * sms) / std::min(1.0, bps / 4.0) /
-                       std::min(1.0, units / groups);
+      const int K = paired && units >= 2.0 * groups ? 2 : 1;
+      const double rounds = std::ceil(units / (groups * K));
+      // a round's clocks per high index: the entries, the step, and the share
+      // of a seed (rows x words) in walks of about rounds / 4 high indices
+      const double work = (double)Bp * ((K == 2 ? 2.5 : 3.8) * d * W + 10.0) + 6.0 * d * W + 60.0 +
+                          1.5 * d * (F - k) * W / std::max(1.0, rounds * K / 4.0);
+      const double t = rounds * K * work * std::max(bps, 3.0);
       cands.push_back({t, S, W, k});
     }
   }
@@ -323,7 +348,10 @@ static bool tc_choose(const int64_t* a, int R, int C, int d, int marginal, const
   auto mine = [&](int steps) {
     return 27.0 + (tiles + std::sqrt((d >= 3 ? 8.0 : 3.0) * tiles)) * std::max(0.55, 0.15 + 0.0345 * steps);
   };
-  if (mine(2) > table) return false;
+  // steps from the low rows' entries: about a feature per unit of them and vector
+  long long units_low = 0;
+  for (int t = 0; t < k * C; ++t) units_low += std::llabs(a[t]);
+  if (mine((int)std::min<long long>(units_low * d / 16, 1000)) > table || units_low * d > 16 * ld::kTcMaxSteps) return false;
   TcLayout lay;
   if (!tc_layout(a, R, C, d, marginal, k, &lay) || mine(lay.steps) > table) return false;
   // with the completion counts of any walk length
@@ -354,17 +382,25 @@ ld_status choose_kernel(const int64_t* a, int R, int C, int d, int marginal, con
     return ld_fail(LD_ERR_ARG, "column_split %d is not -1, 0, 2, 4 or 8", o.column_split);
   if (o.kernel != LD_KERNEL_WIDE && d <= 10 && o.lane_bits != 64 && fits32) {
     const int base = d <= 2 ? 2 : d, F = R - 1;
-    double best_t = 0;
-    bool found = false;
+    // per low-row count only the lane counts are formed (table_config's rules
+    // on running column sums); the chosen one's layout is built once
+    std::vector<long long> sum(C, 0), low(C, 0);
+    for (int i = 0; i < R; ++i)
+      for (int l = 0; l < C; ++l) sum[l] += std::llabs(a[(size_t)i * C + l]);
+    const int HW = o.column_split <= 0 && half_allowed(d, o) ? half_words(d, C, 1) : 0;
+    double best_t = 0, best_half = 0;
+    int best_k = -1, half_k = -1, best_words = 0;
     for (int k = 0; k <= F && o.column_split <= 0; ++k) {
       const unsigned long long B = ipow(base, k);
       if (B > 1024) break;
+      int WB = 0, WA = 0;
+      if (k > 0)
+        for (int l = 0; l < C; ++l) low[l] += std::llabs(a[(size_t)(k - 1) * C + l]);
       if (o.low_rows >= 0 && k != std::min(o.low_rows, F)) continue;
-      Choice c;
-      if (!table_config(a, R, C, d, marginal, k, o.lane_bits, &c)) continue;
-      const int NW = d * c.WT;
+      if (!table_words(sum.data(), low.data(), C, d, marginal, o.lane_bits, &WB, &WA)) continue;
+      const int NW = d * round4(WB + WA);
       if (B * (unsigned long long)NW > (o.low_rows >= 0 ? 16384ull : 8192ull)) continue;
-      const double words = (double)d * (c.WB + c.WA);
+      const double words = (double)d * (WB + WA);
       const double per_lab = words + (2.0 * words + 40.0) / (double)B;
       // parallel units: the high indices, or (d >= 3, label symmetry) the
       // ones that can hold a class minimum; time ~ units * B * per_lab
@@ -375,23 +411,24 @@ ld_status choose_kernel(const int64_t* a, int R, int C, int d, int marginal, con
         if (ld_symmetry_walks(d, F - k, 0, ipow(base, F - k), &pass) == LD_OK && pass > 0) units = (double)pass;
       }
       double t = units * (double)B * per_lab / std::min(units, (double)full_threads);
-      if (!found || t < best_t * 0.999) { best_t = t; *ch = c; found = true; }
+      if (best_k < 0 || t < best_t * 0.999) { best_t = t; best_k = k; best_words = WB + WA; }
       // two columns per word: a word costs 1.1 absolute-difference-accumulates
       // (2.5 against 2.27 clocks, 24 words, paired walks), where those cover
       // one 32-bit or four 8-bit columns
-      const int W = half_allowed(d, o) ? half_words(d, C, 1) : 0;
-      if (W > 0 && 1.1 * W < c.WB + c.WA) {
-        const double hw = 1.1 * d * W + 1.0;
+      if (HW > 0 && 1.1 * HW < WB + WA) {
+        const double hw = 1.1 * d * HW + 1.0;
         t = units * (double)B * (hw + (2.0 * hw + 40.0) / (double)B) / std::min(units, (double)full_threads);
-        if (t < best_t * 0.999 && half_layout(a, R, C, d, marginal, k, W, 1, &c.half)) {
-          best_t = t;
-          c.HW = W;
-          *ch = c;
-        }
+        if (half_k < 0 || t < best_half * 0.999) { best_half = t; half_k = k; }
       }
     }
-    if (found) {
-      tc_choose(a, R, C, d, marginal, o, sms, (ch->HW > 0 ? 1.1 * ch->HW : ch->WB + ch->WA) * d, ch);
+    if (best_k >= 0) {
+      HalfLayout half;
+      const bool use_half = half_k >= 0 && best_half < best_t * 0.999 &&
+                            half_layout(a, R, C, d, marginal, half_k, HW, 1, &half);
+      if (!table_config(a, R, C, d, marginal, use_half ? half_k : best_k, o.lane_bits, ch))
+        return ld_fail(LD_ERR_ARG, "no table kernel for d=%d, %d columns", d, C);
+      if (use_half) { ch->HW = HW; ch->half = std::move(half); }
+      tc_choose(a, R, C, d, marginal, o, sms, (use_half ? 1.1 * HW : best_words) * d, ch);
       return LD_OK;
     }
     // too wide for one thread's registers: S lanes share each high index, in
@@ -648,7 +685,7 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
     // walks costs about a tile (d >= 3: three), and a CTA waits for half a
     // group at the end: of n tiles per CTA, walks of sqrt(2 n) (sqrt(6 n))
     // lose least.
-    const unsigned long long per_thread = D >= 3 ? 4ull : 16ull;
+    const unsigned long long per_thread = D >= 3 || (HW > 0 && S > 1) ? 4ull : 16ull;
     int fw = 0;
     if (tc) {
       const double tiles = (double)walks_run(0, 0, ipow(base, nh)) / ((double)di.sms * 128.0);

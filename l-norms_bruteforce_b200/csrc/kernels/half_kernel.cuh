@@ -62,37 +62,38 @@ __host__ __device__ inline int half_region_words(int D, int W, int R, int Bp) {
   return (R + 3) * half_row_words(W) + Bp * half_entry_words(D, W);
 }
 
+// H[v] += row * m (m = 1, 0 or -1; rows are 16-byte aligned)
 template <int D, int W>
-__device__ __forceinline__ void half_add(uint32_t* H, const uint32_t* row, int v) {
+__device__ __forceinline__ void half_add(uint32_t* H, const uint32_t* row, int v, uint32_t m) {
+  const uint4* r = reinterpret_cast<const uint4*>(row);
 #pragma unroll
-  for (int w = 0; w <= W; ++w) H[v * (W + 1) + w] += row[w];
-}
-template <int D, int W>
-__device__ __forceinline__ void half_sub(uint32_t* H, const uint32_t* row, int v) {
+  for (int q = 0; q < (W + 4) / 4; ++q) {
+    const uint4 x = r[q];
+    const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-  for (int w = 0; w <= W; ++w) H[v * (W + 1) + w] -= row[w];
+    for (int c = 0; c < 4; ++c)
+      if (4 * q + c <= W) H[v * (W + 1) + 4 * q + c] += xs[c] * m;
+  }
 }
 
 // high row `row` moves from label a to label b
 template <int D, int W>
 __device__ __forceinline__ void half_move(uint32_t* H, const uint32_t* row, int a, int b) {
   if constexpr (D == 1) {
-#pragma unroll
-    for (int w = 0; w <= W; ++w) H[w] += b ? 2u * row[w] : 0u - 2u * row[w];
+    half_add<D, W>(H, row, 0, b ? 2u : 0u - 2u);
   } else if constexpr (D == 2) {
-    if (b) half_add<D, W>(H, row, 0); else half_sub<D, W>(H, row, 0);
+    half_add<D, W>(H, row, 0, b ? 1u : 0u - 1u);
   } else {
-    if (a == 1) half_sub<D, W>(H, row, 0);
-    if (a == 2) half_sub<D, W>(H, row, 1);
-    if (b == 1) half_add<D, W>(H, row, 0);
-    if (b == 2) half_add<D, W>(H, row, 1);
-    if (a == 0 && b != 0) half_add<D, W>(H, row, 2);
-    if (a != 0 && b == 0) half_sub<D, W>(H, row, 2);
+    half_add<D, W>(H, row, 0, (uint32_t)(b == 1) - (uint32_t)(a == 1));
+    half_add<D, W>(H, row, 1, (uint32_t)(b == 2) - (uint32_t)(a == 2));
+    half_add<D, W>(H, row, 2, (uint32_t)(b != 0) - (uint32_t)(a != 0));
   }
 }
 
-// register vectors of high index h: every vector starts from sH0 (the bias,
-// for d = 1 with the fixed row)
+// Register vectors of high index h: every vector starts from sH0 (the bias,
+// for d = 1 with the fixed row).  Without branches on the label: the groups of
+// a warp hold different high indices (with branches and word-wise loads a
+// seed of 18 rows of 8 x 16 words took 10,000 clocks).
 template <int D, int W>
 __device__ __forceinline__ void half_seed(uint32_t* H, const uint32_t* sA, const uint32_t* sH0, int k, int nh,
                                           unsigned long long h) {
@@ -101,24 +102,22 @@ __device__ __forceinline__ void half_seed(uint32_t* H, const uint32_t* sA, const
   for (int v = 0; v < P::NR; ++v)
 #pragma unroll
     for (int w = 0; w <= W; ++w) H[v * P::WV + w] = sH0[w];
+  const uint32_t* row = sA + k * P::WT;
   if constexpr (D <= 2) {
-    const unsigned long long g = h ^ (h >> 1);
-    for (int t = 0; t < nh; ++t) {
-      const int lab = (int)((g >> t) & 1ull);
-      const uint32_t* row = sA + (k + t) * P::WT;
-      if (lab) half_add<D, W>(H, row, 0);
-      else if (D == 1) half_sub<D, W>(H, row, 0);
+    unsigned long long g = h ^ (h >> 1);
+    for (int t = 0; t < nh; ++t, g >>= 1, row += P::WT) {
+      const uint32_t lab = (uint32_t)(g & 1ull);
+      half_add<D, W>(H, row, 0, D == 1 ? 2u * lab - 1u : lab);
     }
   } else {
-    unsigned long long q = h;
-    for (int t = 0; t < nh; ++t) {
-      const int r = (int)(q % 6ull);
-      const int lab = r < 3 ? r : 5 - r;
-      q /= 3ull;
-      if (lab == 0) continue;
-      const uint32_t* row = sA + (k + t) * P::WT;
-      half_add<D, W>(H, row, lab - 1);
-      half_add<D, W>(H, row, 2);
+    unsigned long long x = h;
+    for (int t = 0; t < nh; ++t, row += P::WT) {
+      const unsigned long long q = x / 3ull;
+      const unsigned n = (unsigned)(x - 3ull * q), lab = (q & 1ull) ? 2u - n : n;
+      x = q;
+      half_add<D, W>(H, row, 0, lab == 1u);
+      half_add<D, W>(H, row, 1, lab == 2u);
+      half_add<D, W>(H, row, 2, lab != 0u);
     }
   }
 }
