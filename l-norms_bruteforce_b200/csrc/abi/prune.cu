@@ -45,6 +45,14 @@ long long labeling_value(const int64_t* a, int R, int C, int d, int marginal, co
   return v;
 }
 
+// Capacities of the two prefix lists (8 bytes each; the first also holds
+// every walk).
+constexpr unsigned long long kListA = 1ull << 21, kListB = 1ull << 22;
+// Listed prefixes that hold more high indices than this are extended by a part
+// of their rows first: such a level costs about 80 us (the norm of the rows
+// left, a launch, a wait for the count), bounding 2^23 high indices 150.
+constexpr unsigned long long kLevelHighs = 1ull << 23;
+
 // The norm of rows [0, r) alone (every labeling of them), for the bounds:
 // the plain solver on those rows plus a zero fixed row.  Falls back to the
 // always-valid sum of absolute entries when the submatrix is too large to
@@ -107,7 +115,7 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
   const int base = d <= 2 ? 2 : d, F = R - 1;
   Choice ch;
   const void* kb = nullptr;
-  const void* ks = nullptr;
+  const void* ke = nullptr;
   int k = -1;
   for (int kk = std::min(F - 1, 10); kk >= 0 && k < 0; --kk) {
     const unsigned long long B = ipow(base, kk);
@@ -127,13 +135,13 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
     const void* b1; const void* b2;
     ld::prune_kernel_ptrs(d, c.WB, c.WA, &b1, &b2);
     if (!b1 || B * (unsigned long long)(d * c.WT) * 4ull > 48ull * 1024ull) continue;
-    ch = c; kb = b1; ks = b2; k = kk;
+    ch = c; kb = b1; ke = b2; k = kk;
   }
   if (k < 0) return plain();
   const int nh = F - k;
   // walk rows: every walk gets one bound in the first launch, so at most
-  // about 2^21 walks; the surviving walks' high indices are split over the
-  // threads of the scan, so long walks cost nothing extra there
+  // about 2^21 walks; the surviving ones are extended over all threads, so
+  // long walks cost nothing extra there
   int fw = std::min(nh, 5);
   while (fw < nh && (double)(nh - fw) * std::log2((double)base) > 21.0) ++fw;
   const unsigned long long walk_len = ipow(base, fw), walks = ipow(base, nh - fw);
@@ -145,58 +153,62 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
 
   // bounds of the rest rows, in the kernel's representation
   long long m_low = 0, m_walk = 0, kl = 0, kh = 0;
-  st = rest_norm(a, C, d, marginal, k, o.device, &m_low);
-  if (st == LD_OK) st = rest_norm(a, C, d, marginal, k + fw, o.device, &m_walk);
+  st = rest_norm(a, C, d, marginal, k + fw, o.device, &m_walk);
   if (st != LD_OK) return st;
   if (d == 1 && marginal) {
     for (int i = 0; i < R; ++i) { const int64_t v = a[(size_t)i * C]; (i < k ? kl : kh) += v < 0 ? -v : v; }
-    m_low += kl;
     m_walk += kl;
   }
   const long long offset = kh + kl;
   const long long thr = ps.incumbent == LLONG_MIN ? LLONG_MIN : ps.incumbent + offset;
 
-  // image: header | tot | h0 | tb | ttop | thigh | rows
+  // image: header | tot | h0 | tb | the prefix rows' totals | rows
   const int WT = ch.WT;
-  std::vector<int64_t> tot(C, 0), h0(C, 0), tb(C, 0), ttop(C, 0), thigh(C, 0);
+  std::vector<int64_t> tot(C, 0), h0(C, 0), tb(C, 0);
   for (int i = 0; i < R; ++i)
-    for (int l = 0; l < C; ++l) {
-      const int64_t x = a[(size_t)i * C + l];
-      tot[l] += x;
-      if (i >= k) thigh[l] += x;
-      if (i >= k + fw) ttop[l] += x;
-    }
+    for (int l = 0; l < C; ++l) tot[l] += a[(size_t)i * C + l];
   if (d == 1) {
     for (int l = 0; l < C; ++l) h0[l] = a[(size_t)(R - 1) * C + l];
     if (marginal) { h0[0] += kh; tb[0] = -kl; }
   }
-  const size_t offTot = 256, offH0 = 512, offTb = 768, offTtop = 1024, offThigh = 1280, offA = 1536;
+  // totals of the fixed row and the rows above the lowest `rows`, packed
+  auto pack_totals = [&](int rows, uint32_t* out) {
+    std::vector<int64_t> t(C, 0);
+    for (int i = rows; i < R; ++i)
+      for (int l = 0; l < C; ++l) t[l] += a[(size_t)i * C + l];
+    pack_row(t.data(), ch, out);
+  };
+  const size_t offBest = 64, offTot = 256, offH0 = 512, offTb = 768, offTtop = 1024, offA = 1280;
   const size_t upload = offA + (size_t)R * WT * 4;
   std::vector<char> image(upload, 0);
   const long long gmin = LLONG_MIN;
   memcpy(image.data() + 8, &gmin, sizeof gmin);
+  const ld::Slot none{LLONG_MIN, ULLONG_MAX};
+  memcpy(image.data() + offBest, &none, sizeof none);   // then the high indices kept
   pack_row(tot.data(), ch, (uint32_t*)(image.data() + offTot));
   pack_row(h0.data(), ch, (uint32_t*)(image.data() + offH0));
   pack_row(tb.data(), ch, (uint32_t*)(image.data() + offTb));
-  pack_row(ttop.data(), ch, (uint32_t*)(image.data() + offTtop));
-  pack_row(thigh.data(), ch, (uint32_t*)(image.data() + offThigh));
+  pack_totals(k + fw, (uint32_t*)(image.data() + offTtop));
   for (int i = 0; i < R; ++i) pack_row(a + (size_t)i * C, ch, (uint32_t*)(image.data() + offA) + (size_t)i * WT);
 
   const size_t smem_b = (size_t)ld::prune_smem_words(d, WT, R, B, false) * 4;
-  const size_t smem_s = (size_t)ld::prune_smem_words(d, WT, R, B, true) * 4;
-  int bps_b = 0, bps_s = 0;
+  const size_t smem_e = (size_t)ld::prune_smem_words(d, WT, R, B, true) * 4;
+  int bps_b = 0, bps_e = 0;
   if (cudaSetDevice(o.device) != cudaSuccess ||
-      ld_raise_smem_limit(kb, smem_b) != cudaSuccess || ld_raise_smem_limit(ks, smem_s) != cudaSuccess ||
+      ld_raise_smem_limit(kb, smem_b) != cudaSuccess || ld_raise_smem_limit(ke, smem_e) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps_b, kb, ld::kPruneThreads, smem_b) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps_s, ks, ld::kPruneThreads, smem_s) != cudaSuccess ||
-      bps_b < 1 || bps_s < 1)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps_e, ke, ld::kPruneThreads, smem_e) != cudaSuccess ||
+      bps_b < 1 || bps_e < 1)
     return ld_fail(LD_ERR_CUDA, "pruned kernels do not fit an SM");
-  const unsigned long long blocks_b = std::max(1ull, std::min<unsigned long long>((unsigned long long)di.sms * bps_b,
-                                                   (walks + ld::kPruneThreads - 1) / ld::kPruneThreads));
-  const unsigned long long blocks_s = (unsigned long long)di.sms * bps_s;
+  const unsigned long long full_b = (unsigned long long)di.sms * bps_b, blocks_e = (unsigned long long)di.sms * bps_e;
+  // list A: the walks, then every other level's survivors; list B: the levels
+  // between, or the surviving high indices of one launch
+  const unsigned long long capA = std::max(walks, std::min<unsigned long long>(ps.highs_total, kListA));
+  const unsigned long long capB = std::min<unsigned long long>(ps.highs_total, kListB);
   const size_t off_slots = align256(upload);
-  const size_t off_list = off_slots + align256(blocks_s * sizeof(ld::Slot));
-  const size_t off_cnt = off_list + align256(walks * 8);
+  const size_t off_a = off_slots + align256(blocks_e * sizeof(ld::Slot));
+  const size_t off_b = off_a + align256(capA * 8);
+  const size_t off_cnt = off_b + align256(capB * 8);
   const size_t dbytes = off_cnt + 256;
   if (o.device < 0 || o.device >= 64) return ld_fail(LD_ERR_ARG, "device %d out of range", o.device);
   std::lock_guard<std::mutex> lock(g_pws_mu[o.device]);
@@ -207,15 +219,16 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
   if (st != LD_OK) return st;
   char* dmem = (char*)r->dmem;
   cudaStream_t s = r->stream;
-  ld::Slot* out_h = (ld::Slot*)r->hstage;
-  unsigned long long* hstat = (unsigned long long*)((char*)r->hstage + 64);
+  struct Best { ld::Slot slot; unsigned long long kept; };
+  Best* out_h = (Best*)r->hstage;
+  unsigned long long* hcount = (unsigned long long*)((char*)r->hstage + 64);
   float ms_b = 0.f, ms_s = 0.f;
   auto fail = [&](const char* what, cudaError_t e) {
     cudaStreamSynchronize(s);
     return ld_fail(LD_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   };
+  unsigned long long visited = 0, d2h = sizeof(Best);
   cudaError_t e;
-  if ((e = cudaMemsetAsync(dmem + off_cnt, 0, 256, s)) != cudaSuccess) return fail("memset", e);
   if ((e = cudaMemcpyAsync(dmem, image.data(), upload, cudaMemcpyHostToDevice, s)) != cudaSuccess) return fail("upload", e);
   {
     ld::PruneArgs args;
@@ -225,7 +238,7 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
     t.hinit = (const uint32_t*)(dmem + offH0);
     t.tbias = (const uint32_t*)(dmem + offTb);
     t.R = R; t.k = k; t.B = B; t.fw = fw;
-    t.walk_len = walk_len; t.walk_begin = 0; t.walk_end = walks;
+    t.walk_len = walk_len;
     // d = 3: the walk bound also drops walks that hold no class minimum
     t.sym_digits = (d == 3 && !o.enumerate_all && nh - fw > 0) ? nh - fw : 0;
     t.sym_table = nullptr; t.rank_begin = t.rank_end = 0;
@@ -237,43 +250,110 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
     t.red.slots = (ld::Slot*)(dmem + off_slots);
     t.red.work = nullptr;
     args.ttop = (const uint32_t*)(dmem + offTtop);
-    args.thigh = (const uint32_t*)(dmem + offThigh);
     args.threshold = thr;
-    args.m_walk = m_walk;
-    args.m_low = m_low;
-    args.list = (unsigned long long*)(dmem + off_list);
     args.list_count = (unsigned long long*)(dmem + off_cnt);
-    args.stats = (unsigned long long*)(dmem + off_cnt + 8);
+    args.best = (ld::Slot*)(dmem + offBest);
     void* params[] = {&args};
+    // Bound the extensions [begin, end) of the listed prefixes.  Runs of up to
+    // `expand` of them: long ones share the seed of rows x words, but half of
+    // the threads should have one.
+    auto bound = [&](unsigned long long begin, unsigned long long end) -> cudaError_t {
+      const unsigned long long total = end - begin;
+      unsigned long long run = 1;
+      while (run * base <= args.expand && run * base <= 4096 && total / run > full_b * (ld::kPruneThreads / 2))
+        run *= base;
+      args.run = run;
+      t.walk_begin = begin; t.walk_end = end;
+      const unsigned long long need = ((total + run - 1) / run + ld::kPruneThreads - 1) / ld::kPruneThreads;
+      cudaError_t x = cudaMemsetAsync(args.list_count, 0, 8, s);
+      if (x != cudaSuccess) return x;
+      return cudaLaunchKernel(kb, dim3((unsigned)std::min(full_b, need)), dim3(ld::kPruneThreads), params, smem_b, s);
+    };
     if ((e = cudaEventRecord(r->ev0, s)) != cudaSuccess) return fail("event", e);
-    if ((e = cudaLaunchKernel(kb, dim3((unsigned)blocks_b), dim3(ld::kPruneThreads), params, smem_b, s)) != cudaSuccess)
-      return fail("walk bound launch", e);
+    unsigned long long* lists[2] = {(unsigned long long*)(dmem + off_a), (unsigned long long*)(dmem + off_b)};
+    const unsigned long long caps[2] = {capA, capB};
+    int cur = 0;                       // the list that holds the survivors
+    args.src = nullptr; args.expand = walks; args.list = lists[0]; args.m_rest = m_walk;
+    if ((e = bound(0, walks)) != cudaSuccess) return fail("walk bound launch", e);
     if ((e = cudaEventRecord(r->ev1, s)) != cudaSuccess) return fail("event", e);
-    // When more than a quarter of the walks survive their bound the scan
+    if ((e = cudaMemcpyAsync(hcount, args.list_count, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+      return fail("survivors", e);
+    // the low rows' norm, meanwhile
+    if ((st = rest_norm(a, C, d, marginal, k, o.device, &m_low)) != LD_OK) { cudaStreamSynchronize(s); return st; }
+    m_low += kl;
+    if ((e = cudaSetDevice(o.device)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
+      return fail("walk bound", e);
+    unsigned long long n = *hcount;
+    ps.walks_kept = n;
+    d2h += 8;
+    // When more than a quarter of the walks survive their bound the search
     // would do most of the plain enumeration's work at a lower rate: run the
     // plain enumeration instead (same result).
-    if ((e = cudaMemcpyAsync(hstat, dmem + off_cnt, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s)) !=
-        cudaSuccess)
-      return fail("survivors", e);
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail("walk bound", e);
-    if (o.prune_policy == 0 && hstat[0] * 4ull > walks) {
+    if (o.prune_policy == 0 && n * 4ull > walks) {
       cudaEventElapsedTime(&ms_b, r->ev0, r->ev1);
-      ps.walks_kept = hstat[0];
       ps.bound_ms = ms_b;
       return plain();
     }
-    if ((e = cudaLaunchKernel(ks, dim3((unsigned)blocks_s), dim3(ld::kPruneThreads), params, smem_s, s)) != cudaSuccess)
-      return fail("scan launch", e);
+    t.sym_digits = 0;
+    std::vector<uint32_t> tw(WT);
+    for (int left = fw; left > 0;) {
+      // extend by all the rows left, or by a part of them: about half, as many
+      // as the other list takes
+      int more = left;
+      if ((double)n * (double)ipow(base, left) > (double)kLevelHighs) {
+        int m = 0;
+        while (2 * m < left && n * ipow(base, m + 1) <= std::min(kListA, caps[cur ^ 1])) ++m;
+        if (m >= 2) more = m;
+      }
+      left -= more;
+      args.m_rest = m_low;
+      if (left > 0) {
+        if ((st = rest_norm(a, C, d, marginal, k + left, o.device, &args.m_rest)) != LD_OK) return st;
+        args.m_rest += kl;
+        if ((e = cudaSetDevice(o.device)) != cudaSuccess) return fail("device", e);
+      }
+      if (d >= 2) {
+        pack_totals(k + left, tw.data());
+        if ((e = cudaMemcpyAsync(dmem + offTtop, tw.data(), WT * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(s)) != cudaSuccess)
+          return fail("totals", e);
+      }
+      args.src = lists[cur];
+      args.list = lists[cur ^ 1];
+      args.expand = ipow(base, more);
+      t.fw = left;
+      t.walk_len = ipow(base, left);
+      const unsigned long long total = n * args.expand;
+      if (left > 0) {
+        if ((e = bound(0, total)) != cudaSuccess) return fail("level launch", e);
+        if ((e = cudaMemcpyAsync(hcount, args.list_count, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(s)) != cudaSuccess)
+          return fail("level bound", e);
+        n = *hcount;
+        cur ^= 1;
+        d2h += 8;
+        continue;
+      }
+      // whole high indices: as many at once as the list can hold, a power of
+      // the base (runs do not straddle the launches)
+      visited = total;
+      unsigned long long seg = 1;
+      while (seg * base <= caps[cur ^ 1]) seg *= base;
+      for (unsigned long long v = 0; v < total; v += seg) {
+        if ((e = bound(v, std::min(total, v + seg))) != cudaSuccess) return fail("scan launch", e);
+        if ((e = cudaLaunchKernel(ke, dim3((unsigned)blocks_e), dim3(ld::kPruneThreads), params, smem_e, s)) != cudaSuccess)
+          return fail("evaluation launch", e);
+      }
+    }
     if ((e = cudaEventRecord(r->ev2, s)) != cudaSuccess) return fail("event", e);
   }
-  if ((e = cudaMemcpyAsync(out_h, dmem + 16, sizeof(ld::Slot), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+  if ((e = cudaMemcpyAsync(out_h, dmem + offBest, sizeof(Best), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
     return fail("result", e);
-  if ((e = cudaMemcpyAsync(hstat, dmem + off_cnt, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-    return fail("stats", e);
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail("solve", e);
   cudaEventElapsedTime(&ms_b, r->ev0, r->ev1);
   cudaEventElapsedTime(&ms_s, r->ev1, r->ev2);
-  const ld::Slot out = *out_h;
+  const ld::Slot out = out_h->slot;
+  const unsigned long long kept = out_h->kept;
   if (ps.incumbent != LLONG_MIN && out.value < ps.incumbent)
     return ld_fail(LD_ERR_CUDA, "internal: pruned result %lld below the incumbent %lld", (long long)out.value,
                    (long long)ps.incumbent);
@@ -285,13 +365,12 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
   res->kernel_kind = LD_KERNEL_TABLE;
   res->lane_bits = ch.lane_bits;
   res->h2d_bytes = upload;
-  res->d2h_bytes = sizeof out + 4 * sizeof(unsigned long long);
-  res->evaluated = hstat[2] * (unsigned long long)B;   // high indices whose block was scanned
+  res->d2h_bytes = d2h;
+  res->evaluated = kept * (unsigned long long)B;   // high indices whose block was scanned
   if (strategy) ld_gray_labels(out.index, R, d, strategy);
   ps.pruned = 1;
-  ps.walks_kept = hstat[1];
-  ps.highs_kept = hstat[2];
-  ps.highs_visited = hstat[3];
+  ps.highs_kept = kept;
+  ps.highs_visited = visited;
   ps.bound_ms = ms_b;
   ps.scan_ms = ms_s;
   if (stats) *stats = ps;

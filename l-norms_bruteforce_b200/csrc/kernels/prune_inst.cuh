@@ -11,8 +11,8 @@ namespace pinst {
 template <int D, int WB, int WA>
 void put(PruneKernelTab& t) {
   if constexpr (WB + WA > 0) {
-    t[D][WB][WA][0] = (const void*)&walk_bound_kernel<D, WB, WA>;
-    t[D][WB][WA][1] = (const void*)&prune_scan_kernel<D, WB, WA>;
+    t[D][WB][WA][0] = (const void*)&prefix_bound_kernel<D, WB, WA>;
+    t[D][WB][WA][1] = (const void*)&prune_eval_kernel<D, WB, WA>;
   }
 }
 template <int D, int WB, int... I>

@@ -8,15 +8,19 @@
 //     value <= sum_ml |P_ml| + max over the rest's labelings of sum_ml |Q_ml|
 // and the second term is exactly the L_d norm (for LM: the marginal norm)
 // of the rest rows alone, computed beforehand by the plain solver.  The
-// search runs in two launches:
-//   1. walk_bound_kernel: for every walk, the bound with P over the top rows
+// search goes from short prefixes to whole high indices:
+//   1. prefix_bound_kernel: for every walk, the bound with P over the top rows
 //      and the rest = walk + low rows; walks whose bound is below the
 //      incumbent are dropped, the others are appended to a list;
-//   2. prune_scan_kernel: every listed walk is walked as in the table kernel;
-//      for every high index h the bound with P = H(h) and the rest = the low
-//      rows decides whether its B labelings need evaluating, and the
-//      surviving h are evaluated by the whole warp together (H broadcast by
-//      shuffles, the B table entries split over the lanes).
+//   2. prefix_bound_kernel again: every listed prefix is extended by some walk
+//      rows and bounded with the norm of the rows that remain, while the
+//      listed ones hold many high indices, and at last by all of them, when
+//      the rest is the low rows.  (One step from the walks to their high
+//      indices took 2214 us for a 44 x 44 matrix whose 9037 listed walks hold
+//      148 M of them; one more level leaves 5.6 M.)
+//   3. prune_eval_kernel: the B labelings of each surviving high index, each
+//      table shared by a few threads.  Survivors lie close together: evaluated
+//      where they are found, 1075 of them kept one warp busy for 50 us.
 // Only bounds strictly below the incumbent prune, so every labeling that
 // attains the maximum is evaluated and the smallest Gray index among them is
 // the one reported: the result equals the plain enumeration's.
@@ -32,15 +36,17 @@
 namespace ld {
 
 struct PruneArgs {
-  TableArgs t;                    // the table kernel's operands (walk range = all walks)
-  const uint32_t* ttop;           // WT words: column totals of the fixed + top rows (d >= 2)
-  const uint32_t* thigh;          // WT words: column totals of the fixed + top + walk rows (d >= 2)
+  TableArgs t;                    // the table kernel's operands; fw = rows below a prefix, walk_begin ..
+                                  // walk_end = the extensions to bound
+  const uint32_t* ttop;           // WT words: column totals of the fixed + prefix rows (d >= 2)
   long long threshold;            // incumbent, in the kernel's value representation
-  long long m_walk;               // norm of the walk + low rows (representation-adjusted)
-  long long m_low;                // norm of the low rows (representation-adjusted)
-  unsigned long long* list;       // surviving walk indices
-  unsigned long long* list_count; // number of surviving walks
-  unsigned long long* stats;      // [0] walks kept, [1] h kept, [2] h visited
+  long long m_rest;               // norm of the rows below a prefix (representation-adjusted)
+  const unsigned long long* src;  // the listed prefixes to extend (null: extension = prefix)
+  unsigned long long expand;      // extensions of each, a power of the base
+  unsigned long long run;         // consecutive extensions per thread, a power of the base up to it
+  unsigned long long* list;       // surviving prefixes (evaluation: high indices)
+  unsigned long long* list_count; // their number
+  Slot* best;                     // evaluation: the best over its launches; then the high indices seen
 };
 
 constexpr int kPruneThreads = 128;
@@ -51,25 +57,66 @@ template <int D, int WB, int WA>
 __device__ __forceinline__ long long prefix_abs(const uint32_t* H, const uint32_t* T) {
   using S = Shape<D, WB, WA>;
   static_assert(D != 3 || S::NR == 3, "pruned d = 3 shapes keep H1 + H2 in registers");
-  uint32_t acc = 0u;
+  uint32_t acc[2] = {0u, 0u};   // two chains: the launches have few warps
   if (D == 1) {
 #pragma unroll
-    for (int w = 0; w < S::WV; ++w) acc = wsad<WB>(w, H[w], 0u, acc);
+    for (int w = 0; w < S::WV; ++w) acc[w & 1] = wsad<WB>(w, H[w], 0u, acc[w & 1]);
   } else if (D == 2) {
 #pragma unroll
     for (int w = 0; w < S::WV; ++w) {
-      acc = wsad<WB>(w, H[w], 0u, acc);
-      acc = wsad<WB>(w, H[w], T[w], acc);
+      acc[0] = wsad<WB>(w, H[w], 0u, acc[0]);
+      acc[1] = wsad<WB>(w, H[w], T[w], acc[1]);
     }
   } else {
 #pragma unroll
     for (int w = 0; w < S::WV; ++w) {
-      acc = wsad<WB>(w, H[w], 0u, acc);
-      acc = wsad<WB>(w, H[S::WV + w], 0u, acc);
-      acc = wsad<WB>(w, H[2 * S::WV + w], T[w], acc);
+      acc[0] = wsad<WB>(w, H[w], 0u, acc[0]);
+      acc[1] = wsad<WB>(w, H[S::WV + w], 0u, acc[1]);
+      acc[w & 1] = wsad<WB>(w, H[2 * S::WV + w], T[w], acc[w & 1]);
     }
   }
-  return (long long)acc;
+  return (long long)(acc[0] + acc[1]);
+}
+
+// H[vec] += row * m, m = -2 .. 2: without a branch on the label, which differs
+// between the lanes of a warp, and with 16-byte loads (one 4-byte load per word
+// and a branch per label made a step of 44 words 590 clocks per warp)
+template <int D, int WB, int WA>
+__device__ __forceinline__ void add_times(uint32_t* H, const uint32_t* row, int vec, int m) {
+  using S = Shape<D, WB, WA>;
+  const uint4* r = reinterpret_cast<const uint4*>(row);
+#pragma unroll
+  for (int q = 0; q < S::WT / 4; ++q) {
+    const uint4 x = r[q];
+    const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int w = 4 * q + c;
+      if (w >= S::WV) continue;
+      uint32_t& h = H[vec * S::WV + w];
+      if (w < WB) {
+        h += xs[c] * (uint32_t)m;
+      } else {
+        uint32_t y = m == 0 ? 0u : m == 2 || m == -2 ? wadd<WB>(w, xs[c], xs[c]) : xs[c];
+        if (m < 0) y = wsub<WB>(w, 0u, y);
+        h = wadd<WB>(w, h, y);
+      }
+    }
+  }
+}
+
+// a row moves from label a to label b (a = -1: it gets its first label)
+template <int D, int WB, int WA>
+__device__ __forceinline__ void relabel(uint32_t* H, const uint32_t* row, int a, int b) {
+  if constexpr (D == 1) {
+    add_times<D, WB, WA>(H, row, 0, a < 0 ? (b ? 1 : -1) : (b ? 2 : -2));
+  } else if constexpr (D == 2) {
+    add_times<D, WB, WA>(H, row, 0, (b == 1) - (a == 1));
+  } else {
+    add_times<D, WB, WA>(H, row, 0, (b == 1) - (a == 1));
+    add_times<D, WB, WA>(H, row, 1, (b == 2) - (a == 2));
+    add_times<D, WB, WA>(H, row, 2, (b > 0) - (a > 0));
+  }
 }
 
 // H over the fixed row and the top rows only (digits fw.. of the high index)
@@ -83,50 +130,16 @@ __device__ __forceinline__ void seed_top(uint32_t* H, const uint32_t* sA, const 
   for (int v = 1; v < S::NR; ++v)
 #pragma unroll
     for (int w = 0; w < S::WV; ++w) H[v * S::WV + w] = 0u;
-  if (D <= 2) {
+  if constexpr (D <= 2) {
     const unsigned long long g = h ^ (h >> 1);
-    for (int t = fw; t < nh; ++t) {
-      const int lab = (int)((g >> t) & 1ull);
-      const uint32_t* row = sA + (k + t) * S::WT;
-      if (D == 1) { if (lab) add_row<D, WB, WA>(H, row, 0); else sub_row<D, WB, WA>(H, row, 0); }
-      else if (lab) add_row<D, WB, WA>(H, row, 0);
-    }
+    for (int t = fw; t < nh; ++t) relabel<D, WB, WA>(H, sA + (k + t) * S::WT, -1, (int)((g >> t) & 1ull));
   } else {
     unsigned long long q = h;
     for (int t = 0; t < fw; ++t) q /= 3ull;
     for (int t = fw; t < nh; ++t) {
       const int r = (int)(q % 6ull);
-      const int lab = r < 3 ? r : 5 - r;
       q /= 3ull;
-      const uint32_t* row = sA + (k + t) * S::WT;
-      if (lab == 1) { add_row<D, WB, WA>(H, row, 0); if (S::NR == 3) add_row<D, WB, WA>(H, row, 2); }
-      else if (lab == 2) { add_row<D, WB, WA>(H, row, 1); if (S::NR == 3) add_row<D, WB, WA>(H, row, 2); }
-    }
-  }
-}
-
-// add the walk rows (digits 0..fw-1) of high index h to a top-row vector
-template <int D, int WB, int WA>
-__device__ __forceinline__ void add_walk_rows(uint32_t* H, const uint32_t* sA, int k, int fw,
-                                              unsigned long long h) {
-  using S = Shape<D, WB, WA>;
-  if (D <= 2) {
-    const unsigned long long g = h ^ (h >> 1);
-    for (int t = 0; t < fw; ++t) {
-      const int lab = (int)((g >> t) & 1ull);
-      const uint32_t* row = sA + (k + t) * S::WT;
-      if (D == 1) { if (lab) add_row<D, WB, WA>(H, row, 0); else sub_row<D, WB, WA>(H, row, 0); }
-      else if (lab) add_row<D, WB, WA>(H, row, 0);
-    }
-  } else {
-    unsigned long long q = h;
-    for (int t = 0; t < fw; ++t) {
-      const int r = (int)(q % 6ull);
-      const int lab = r < 3 ? r : 5 - r;
-      q /= 3ull;
-      const uint32_t* row = sA + (k + t) * S::WT;
-      if (lab == 1) { add_row<D, WB, WA>(H, row, 0); if (S::NR == 3) add_row<D, WB, WA>(H, row, 2); }
-      else if (lab == 2) { add_row<D, WB, WA>(H, row, 1); if (S::NR == 3) add_row<D, WB, WA>(H, row, 2); }
+      relabel<D, WB, WA>(H, sA + (k + t) * S::WT, -1, r < 3 ? r : 5 - r);
     }
   }
 }
@@ -143,18 +156,16 @@ __device__ __forceinline__ void stage(const PruneArgs& args, uint32_t* smem, boo
   uint32_t* sH0 = sTot + WT;
   uint32_t* sTb = sH0 + WT;
   uint32_t* sTtop = sTb + WT;
-  uint32_t* sThigh = sTtop + WT;
   for (int t = threadIdx.x; t < R * WT; t += blockDim.x) sA[t] = ta.A[t];
   for (int t = threadIdx.x; t < WT; t += blockDim.x) {
     sTot[t] = ta.tot[t];
     sH0[t] = ta.hinit[t];
     sTb[t] = ta.tbias ? ta.tbias[t] : 0u;
     sTtop[t] = args.ttop[t];
-    sThigh[t] = args.thigh[t];
   }
   __syncthreads();
   if (!with_table) return;
-  uint32_t* sT = smem + (((R * WT + 5 * WT) + 3) & ~3);
+  uint32_t* sT = smem + (((R * WT + 4 * WT) + 3) & ~3);
   const int k = ta.k, B = ta.B;
   for (int j = threadIdx.x; j < B; j += blockDim.x) {
     uint32_t L1[S::WV], L2[S::WV];
@@ -213,19 +224,20 @@ __device__ __forceinline__ void stage(const PruneArgs& args, uint32_t* smem, boo
 }
 
 __host__ __device__ inline int prune_smem_words(int D, int W, int R, int B, bool with_table) {
-  int head = R * W + 5 * W;
+  int head = R * W + 4 * W;
   head = (head + 3) & ~3;
   return head + (with_table ? B * D * W : 0);
 }
 
-// Launch 1: bound every walk's top-row prefix; list the walks that survive.
-// Each thread takes a contiguous run of walk indices and visits them in
-// order: the top rows' labels are the reflected Gray code of the walk index
-// (binary for d <= 2, 3-ary for d = 3), so consecutive walks differ in one
-// top row, and the prefix vector is seeded once per run and then updated by
-// one row move per walk.
+// Bound prefixes; list those that survive.  A thread takes runs of consecutive
+// prefixes and visits each run in order: the labels of a prefix's rows are its
+// reflected Gray code (binary for d <= 2, 3-ary for d = 3), so consecutive
+// prefixes differ in one row, and the prefix vector is seeded once per run and
+// then updated by one row move per prefix.  Runs are aligned powers of the
+// base, so that the row that moves depends on the step alone and its words are
+// read once for the warp.
 template <int D, int WB, int WA>
-__global__ void __launch_bounds__(kPruneThreads) walk_bound_kernel(const PruneArgs args) {
+__global__ void __launch_bounds__(kPruneThreads) prefix_bound_kernel(const PruneArgs args) {
   using S = Shape<D, WB, WA>;
   extern __shared__ __align__(16) uint32_t smem[];
   stage<D, WB, WA>(args, smem, false);
@@ -234,162 +246,116 @@ __global__ void __launch_bounds__(kPruneThreads) walk_bound_kernel(const PruneAr
   const uint32_t* sA = smem;
   const uint32_t* sH0 = smem + R * S::WT + S::WT;
   const uint32_t* sTtop = smem + R * S::WT + 3 * S::WT;
-  const unsigned long long T = (unsigned long long)gridDim.x * blockDim.x;
-  const unsigned long long tid = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
-  unsigned long long kept = 0;
-  // every lane of a warp runs the same number of iterations (ballots below)
-  const unsigned long long nw = ta.walk_end - ta.walk_begin;
-  const unsigned long long run = (nw + T - 1) / T;
-  const unsigned long long first = ta.walk_begin + tid * run;
+  const unsigned run = (unsigned)args.run;
+  const unsigned long long E = args.expand;
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x * run;
   uint32_t H[S::NR * S::WV];
   // d = 3 with label symmetry: a walk that holds no smallest index of a
   // class (walk_holds_class_min, table_kernel.cuh) is dropped as well
   const int P = D == 3 ? ta.sym_digits : 0;
   unsigned long long pw = 1ull;
   for (int t = 1; t < P; ++t) pw *= 3ull;
-  for (unsigned long long r = 0; r < run; ++r) {
-    const unsigned long long wk = first + r;
-    bool keep = false;
-    if (wk < ta.walk_end) {
-      if (r == 0) {
-        seed_top<D, WB, WA>(H, sA, sH0, k, fw, nh, wk * ta.walk_len);
-      } else {
-        // the one top row whose label differs between walks wk - 1 and wk
-        int i, a, b;
-        if (D <= 2) {
-          i = __ffsll((long long)wk) - 1;
-          b = (int)(((wk >> (i + 1)) & 1ull) ^ 1ull);
-          a = b ^ 1;
+  // every lane of a warp runs the same number of iterations (ballots below)
+  const unsigned long long base = ta.walk_begin + ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x - lane) * run;
+  for (unsigned long long b0 = base; b0 < ta.walk_end; b0 += stride) {
+    const unsigned long long v = b0 + (unsigned long long)lane * run;
+    const bool on = v < ta.walk_end;
+    unsigned long long w0 = on ? v : 0ull;
+    if (args.src) {
+      const unsigned long long slot = w0 / E;
+      w0 = args.src[slot] * E + (w0 - slot * E);
+    }
+    seed_top<D, WB, WA>(H, sA, sH0, k, fw, nh, w0 * ta.walk_len);
+    for (unsigned r = 0; r < run; ++r) {
+      const unsigned long long wk = w0 + r;
+      if (r) {
+        int i;
+        if constexpr (D <= 2) {
+          i = __ffs((int)r) - 1;
+          const int b = ((wk >> (i + 1)) & 1ull) == 0ull;
+          relabel<D, WB, WA>(H, sA + (k + fw + i) * S::WT, b ^ 1, b);
         } else {
-          unsigned long long q = wk;
+          // runs start at multiples of a power of 3, an odd number, so w0
+          // adds its own parity to the digits above the changing one
+          unsigned q = r;
           i = 0;
-          while (q % 3ull == 0ull) { q /= 3ull; ++i; }
-          const int c = (int)(q % 3ull);
-          const int par = (int)((q / 3ull) & 1ull);
-          b = par ? 2 - c : c;
-          a = par ? 3 - c : c - 1;
+          while (q % 3u == 0u) { q /= 3u; ++i; }
+          const int c = (int)(q % 3u);
+          const int par = (int)(((unsigned)w0 ^ (q / 3u)) & 1u);
+          const int b = par ? 2 - c : c, a = par ? 3 - c : c - 1;
+          relabel<D, WB, WA>(H, sA + (k + fw + i) * S::WT, a, b);
         }
-        move_row<D, WB, WA>(H, sA + (k + fw + i) * S::WT, a, b);
       }
-      keep = prefix_abs<D, WB, WA>(H, sTtop) + args.m_walk >= args.threshold;
+      bool keep = on && prefix_abs<D, WB, WA>(H, sTtop) + args.m_rest >= args.threshold;
       if constexpr (D == 3) {
         if (P > 0 && keep) keep = walk_holds_class_min<3>(wk, P, pw);
       }
+      const unsigned mask = __ballot_sync(0xffffffffu, keep);
+      if (mask) {
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(args.list_count, (unsigned long long)__popc(mask));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (keep) args.list[at + __popc(mask & ((1u << lane) - 1u))] = wk;
+      }
     }
-    const unsigned mask = __ballot_sync(0xffffffffu, keep);
-    if (mask) {
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(args.list_count, (unsigned long long)__popc(mask));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (keep) args.list[base + __popc(mask & ((1u << lane) - 1u))] = wk;
-    }
-    kept += keep ? 1ull : 0ull;
   }
-  if (kept) atomicAdd(&args.stats[0], kept);
 }
 
-// Launch 2: walk the listed walks; bound each high index; evaluate the
-// surviving ones with the whole warp.
+// Evaluate the listed high indices: a thread per high index and part of the
+// table, as many parts (at most 32, at least four entries each) as there are
+// threads for; the lanes of a warp share a part, so that an entry is read once
+// for all of them.
 template <int D, int WB, int WA>
-__global__ void __launch_bounds__(kPruneThreads) prune_scan_kernel(const PruneArgs args) {
+__global__ void __launch_bounds__(kPruneThreads) prune_eval_kernel(const PruneArgs args) {
   using S = Shape<D, WB, WA>;
-  constexpr int WT = S::WT, NW = S::NW, NREG = S::NR * S::WV;
+  constexpr int WT = S::WT, NW = S::NW;
   extern __shared__ __align__(16) uint32_t smem[];
-  stage<D, WB, WA>(args, smem, true);
   const TableArgs& ta = args.t;
-  const int R = ta.R, k = ta.k, B = ta.B, fw = ta.fw, nh = R - 1 - k;
-  const uint32_t* sA = smem;
-  const uint32_t* sH0 = smem + R * WT + WT;
-  const uint32_t* sThigh = smem + R * WT + 4 * WT;
-  const uint32_t* sT = smem + (((R * WT + 5 * WT) + 3) & ~3);
-  const unsigned long long T = (unsigned long long)gridDim.x * blockDim.x;
-  const unsigned long long tid = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  const unsigned long long WL = ta.walk_len;
-  const unsigned long long nlist = *args.list_count;
-  // Few surviving walks would leave most threads idle, so each walk is cut
-  // into `split` parts of PL consecutive high indices (at least 8 each), one
-  // part per thread; every part is seeded directly and then walked.
-  unsigned long long split = nlist ? T / nlist : 1ull;
-  const unsigned long long max_split = WL >= 16ull ? WL / 8ull : 1ull;
-  split = split < 1ull ? 1ull : (split > max_split ? max_split : split);
-  const unsigned long long PL = (WL + split - 1) / split;
-  const unsigned long long items = nlist * split;
-  const unsigned long long rounds = (items + T - 1) / T;
+  const unsigned long long n = *args.list_count;
+  const unsigned long long warps = (unsigned long long)gridDim.x * (kPruneThreads / 32);
+  const int B = ta.B, R = ta.R, k = ta.k, nh = R - 1 - k;
+  unsigned P = 1u;
+  while (P < 32u && 8 * (int)P <= B && ((n + 31) / 32) * (2 * P) <= warps) P *= 2u;
   long long bv = LLONG_MIN;
   unsigned long long bn = ULLONG_MAX;
-  unsigned long long hk = 0, hv = 0;
-  uint32_t H[NREG];
-  for (unsigned long long r = 0; r < rounds; ++r) {
-    const unsigned long long item = tid + r * T;
-    const unsigned long long slot = item / split, part = item % split;
-    const unsigned long long u0 = part * PL;
-    const bool live = item < items && u0 < WL;
-    const unsigned long long wk = live ? args.list[slot] : 0ull;
-    const unsigned long long h0 = wk * WL;
-    const unsigned long long u1 = live ? (u0 + PL < WL ? u0 + PL : WL) : 0ull;
-    if (live) {
-      seed_top<D, WB, WA>(H, sA, sH0, k, fw, nh, h0);
-      add_walk_rows<D, WB, WA>(H, sA, k, fw, h0 + u0);
+  // a block without work stages nothing
+  if (((unsigned long long)blockIdx.x * (kPruneThreads / 32)) / P * 32ull < n) {
+    stage<D, WB, WA>(args, smem, true);
+    const uint32_t* sA = smem;
+    const uint32_t* sH0 = smem + R * WT + WT;
+    const uint32_t* sT = smem + (((R * WT + 4 * WT) + 3) & ~3);
+    const unsigned long long warp = (unsigned long long)blockIdx.x * (kPruneThreads / 32) + (threadIdx.x >> 5);
+    const int part = (int)(warp % P), per = (B + (int)P - 1) / (int)P;
+    const int j0 = part * per, j1 = j0 + per < B ? j0 + per : B;
+    uint32_t H[S::NR * S::WV];
+    int best = INT_MIN;
+    unsigned long long best_h = 0ull, last_h = 0ull;
+    if (warp < warps / P * P && j0 < j1) {
+      for (unsigned long long i = warp / P * 32ull + (threadIdx.x & 31); i < n; i += warps / P * 32ull) {
+        const unsigned long long h = args.list[i];
+        seed_top<D, WB, WA>(H, sA, sH0, k, 0, nh, h);
+        int m = INT_MIN;
+        for (int j = j0; j < j1; ++j) m = max(m, entry_value<D, WB, WA>(H, sT + j * NW));
+        if (m > best || (m == best && h < best_h)) { best = m; best_h = h; }
+        last_h = h;
+      }
     }
-    for (unsigned long long uu = 0; uu < PL; ++uu) {
-      const unsigned long long u = u0 + uu;
-      const bool on = live && u < u1;
-      const unsigned long long h = h0 + u;
-      if (on && uu) {
-        int i, a, b;
-        if (D <= 2) {
-          i = __ffsll((long long)u) - 1;
-          b = (int)(((h >> (i + 1)) & 1ull) ^ 1ull);
-          a = b ^ 1;
-        } else {
-          unsigned long long q = u;
-          i = 0;
-          while (q % 3ull == 0ull) { q /= 3ull; ++i; }
-          const int c = (int)(q % 3ull);
-          const int par = (int)((wk ^ (q / 3ull)) & 1ull);
-          b = par ? 2 - c : c;
-          a = par ? 3 - c : c - 1;
-        }
-        move_row<D, WB, WA>(H, sA + (k + i) * WT, a, b);
-      }
-      const bool scan = on && prefix_abs<D, WB, WA>(H, sThigh) + args.m_low >= args.threshold;
-      hv += on ? 1ull : 0ull;
-      hk += scan ? 1ull : 0ull;
-      unsigned mask = __ballot_sync(0xffffffffu, scan);
-      while (mask) {
-        const int src = __ffs(mask) - 1;
-        mask &= mask - 1u;
-        uint32_t Hs[NREG];
-#pragma unroll
-        for (int w = 0; w < NREG; ++w) Hs[w] = __shfl_sync(0xffffffffu, H[w], src);
-        const unsigned long long hs = __shfl_sync(0xffffffffu, h, src);
-        const bool rev = (hs & 1ull) != 0ull;
-        int lv = INT_MIN, ljj = INT_MAX;
-        for (int jj = lane; jj < B; jj += 32) {
-          const int je = rev ? B - 1 - jj : jj;
-          const int v = entry_value<D, WB, WA>(Hs, sT + je * NW);
-          if (v > lv) { lv = v; ljj = jj; }
-        }
-        // warp max of the value, then the smallest position attaining it
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          const int ov = __shfl_xor_sync(0xffffffffu, lv, off);
-          const int oj = __shfl_xor_sync(0xffffffffu, ljj, off);
-          if (ov > lv || (ov == lv && oj < ljj)) { lv = ov; ljj = oj; }
-        }
-        if (lane == src) {
-          const long long v = (long long)lv - ta.value_offset;
-          const unsigned long long n = hs * (unsigned long long)B + (unsigned long long)ljj;
-          if (better(v, n, bv, bn)) { bv = v; bn = n; }
-        }
-      }
+    if (best != INT_MIN) {   // the part's first position attaining it (read backwards for odd h)
+      if (best_h != last_h) seed_top<D, WB, WA>(H, sA, sH0, k, 0, nh, best_h);
+      const bool rev = (best_h & 1ull) != 0ull;
+      int jbest = INT_MAX;
+      for (int j = j0; j < j1; ++j)
+        if (entry_value<D, WB, WA>(H, sT + j * NW) == best) jbest = min(jbest, rev ? B - 1 - j : j);
+      bv = (long long)best - ta.value_offset;
+      bn = best_h * (unsigned long long)B + (unsigned long long)jbest;
     }
   }
-  if (hk) atomicAdd(&args.stats[1], hk);
-  if (hv) atomicAdd(&args.stats[2], hv);
-  grid_reduce(bv, bn, ta.red);
+  if (grid_reduce(bv, bn, ta.red) && threadIdx.x == 0) {
+    const Slot r = *ta.red.result;
+    if (better(r.value, r.index, args.best->value, args.best->index)) *args.best = r;
+    *reinterpret_cast<unsigned long long*>(args.best + 1) += n;
+  }
 }
 
 }  // namespace ld

@@ -38,15 +38,15 @@ const void* table_kernel_pair_ptr(int D, int WB, int WA, int lin);
 const void* table_kernel_lin_ptr(int WB, int WA);
 // all columns in one lane width: PK = 1 (int32, W words) or 4 (int8x4, W words)
 const void* table_kernel_ptr(int D, int W, int PK);
-// pruned-search kernels {walk_bound_kernel, prune_scan_kernel} for (D, WB, WA):
+// pruned-search kernels {prefix_bound_kernel, prune_eval_kernel} for (D, WB, WA):
 //   D = 1: WB <= 2 with WA <= 16, WB in 4, 8, .., 64 with WA = 0
 //   D = 2: WB in 4, 8, .., 48 (WA = 0) or WA in 4, 8, .., 32 (WB = 0)
 //   D = 3: WB in 4, 8, .., 32 (WA = 0) or WA in 4, 8, .., 32 (WB = 0)
 using PruneKernelTab = const void* [4][65][33][2];
 void prune_register_d1(PruneKernelTab& t);
 void prune_register_d23(PruneKernelTab& t);
-// {nullptr, nullptr} when not instantiated
-void prune_kernel_ptrs(int D, int WB, int WA, const void** bound, const void** scan);
+// both null when not instantiated
+void prune_kernel_ptrs(int D, int WB, int WA, const void** bound, const void** eval);
 // batch_table_kernel<D, WB, WA> for the batch lane classes (batch_inst.cu), and
 // the per-matrix fold kernel
 const void* batch_kernel_ptr(int D, int WB, int WA);

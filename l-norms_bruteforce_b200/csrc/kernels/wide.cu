@@ -117,11 +117,11 @@ static const PruneKernelTab& prune_kernels() {
   return tab;
 }
 
-void prune_kernel_ptrs(int D, int WB, int WA, const void** bound, const void** scan) {
-  *bound = *scan = nullptr;
+void prune_kernel_ptrs(int D, int WB, int WA, const void** bound, const void** eval) {
+  *bound = *eval = nullptr;
   if (D < 1 || D > 3 || WB < 0 || WB > 64 || WA < 0 || WA > 32) return;
   *bound = prune_kernels()[D][WB][WA][0];
-  *scan = prune_kernels()[D][WB][WA][1];
+  *eval = prune_kernels()[D][WB][WA][1];
 }
 
 template <typename IT, bool MULTI, bool SYM>

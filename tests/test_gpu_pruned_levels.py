@@ -1,0 +1,47 @@
+"""Pruned search over several levels of prefixes and over several launches of
+high indices: the answers are those of the plain enumeration, which is itself
+checked against the oracle."""
+import numpy as np
+import pytest
+
+import oracle_ffi as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(rng, rows, cols, kind):
+    if kind == "lowrank":
+        a = 5 * rng.standard_normal((rows, 3)) @ rng.standard_normal((3, cols))
+        return np.rint(a).astype(np.int64) + rng.integers(-1, 2, size=(rows, cols))
+    return rng.integers(-kind, kind + 1, size=(rows, cols)).astype(np.int64)
+
+
+@pytest.mark.parametrize("rows,cols,d,marg,kind", [
+    (38, 44, 1, False, "lowrank"),   # 32-bit lanes, an extended level
+    (36, 40, 1, True, "lowrank"),
+    (34, 12, 1, False, 1),           # 8-bit lanes
+    (33, 17, 2, False, "lowrank"),
+    (34, 9, 2, False, 1),
+    (21, 13, 3, False, "lowrank"),
+    (12, 64, 1, False, 40),          # a single prefix
+])
+def test_levels(ld, rows, cols, d, marg, kind):
+    rng = np.random.default_rng(rows * 100 + cols)
+    a = _matrix(rng, rows, cols, kind)
+    plain = ld.solve_reduced(a, d, marg)
+    vals, labs = ld.local_search(a, d, marg, n_random=16, seed=2)
+    for lab in (labs[int(np.argmax(vals))], labs[int(np.argmin(vals))], O.labels(plain.gray_index, rows, d)):
+        sol, st = ld.solve_pruned(a, d, marg, lab, ld.options(prune_policy=1))
+        assert (sol.value, sol.gray_index) == (plain.value, plain.gray_index), st
+        assert st["pruned"] == 1 and st["highs_kept"] <= st["highs_visited"] <= st["highs_total"]
+
+
+@pytest.mark.parametrize("rows,cols,d", [(32, 7, 1), (31, 5, 2), (19, 4, 3)])
+def test_everything_survives(ld, rows, cols, d):
+    """Without an incumbent nothing is dropped: the high indices are bounded
+    and evaluated in several launches."""
+    a = _matrix(np.random.default_rng(rows), rows, cols, 9)
+    plain = ld.solve_reduced(a, d)
+    sol, st = ld.solve_pruned(a, d, False, None, ld.options(prune_policy=1, enumerate_all=1))
+    assert (sol.value, sol.gray_index) == (plain.value, plain.gray_index)
+    assert st["highs_kept"] == st["highs_visited"] == st["highs_total"]
