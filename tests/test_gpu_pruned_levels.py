@@ -1,6 +1,7 @@
 """Pruned search over several levels of prefixes and over several launches of
-high indices: the answers are those of the plain enumeration, which is itself
-checked against the oracle."""
+high indices, and the local search's two integer widths: the answers are those
+of the plain enumeration (itself checked against the oracle) and of the same
+moves made one by one in Python."""
 import numpy as np
 import pytest
 
@@ -45,3 +46,31 @@ def test_everything_survives(ld, rows, cols, d):
     sol, st = ld.solve_pruned(a, d, False, None, ld.options(prune_policy=1, enumerate_all=1))
     assert (sol.value, sol.gray_index) == (plain.value, plain.gray_index)
     assert st["highs_kept"] == st["highs_visited"] == st["highs_total"]
+
+
+def _climb(a, d, marg, lab):
+    """Steepest single-row moves; ties to the smallest row, then label."""
+    lab = list(lab)
+    while True:
+        now, best = O.value(a, d, marg, lab), None
+        for i in range(len(lab)):
+            for t in range(2 if d == 1 else d):
+                if t == lab[i]:
+                    continue
+                g = O.value(a, d, marg, lab[:i] + [t] + lab[i + 1:]) - now
+                if g > 0 and (best is None or g > best[0]):
+                    best = (g, i, t)
+        if best is None:
+            return now, lab
+        lab[best[1]] = best[2]
+
+
+@pytest.mark.parametrize("scale", [1, 10 ** 9])   # int32 and int64 sums
+@pytest.mark.parametrize("rows,cols,d,marg", [(2, 1, 1, False), (9, 33, 1, True), (17, 16, 2, False), (13, 20, 3, False)])
+def test_local_search_moves(ld, rows, cols, d, marg, scale):
+    rng = np.random.default_rng(rows)
+    a = rng.integers(-3, 4, size=(rows, cols)).astype(np.int64) * scale
+    starts = rng.integers(0, 2 if d == 1 else d, size=(5, rows - 1))
+    vals, labs = ld.local_search(a, d, marg, starts=starts)
+    for s, v, lab in zip(starts, vals, labs):
+        assert (int(v), lab.tolist()) == _climb(a, d, marg, [int(x) for x in s])
