@@ -614,7 +614,7 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
     ld::Slot* res = (ld::Slot*)(b->dmem + b->off_res);
     int n = count;
     void* params[] = {(void*)&cres, (void*)&ranges, (void*)&n, (void*)&res};
-    e = cudaLaunchKernel(ld::batch_fold_kernel_ptr(), dim3((count + 127) / 128), dim3(128), params, 0, s);
+    e = cudaLaunchKernel(ld::batch_fold_kernel_ptr(), dim3((count + 3) / 4), dim3(128), params, 0, s);
   }
   for (int p = 0; p < count && e == cudaSuccess; ++p)
     if (b->plans[p])

@@ -81,21 +81,21 @@ __global__ void __launch_bounds__(kBatchMaxThreads, half_min_blocks(D, W, 1, D <
     }
     long long bv = LLONG_MIN;
     unsigned long long bn = ULLONG_MAX;
+    block_top(best, best_h);
     if (best != INT_MIN) {
       half_seed<D, W>(H[0], sA, sH0, k, nh, best_h);
       const int sh = half_sh<D, W>(H[0]);
       const bool rev = (best_h & 1ull) != 0ull;
-      for (int jj = 0; jj < B; ++jj) {
+      int jbest = INT_MAX;
+      for (int je = threadIdx.x; je < B; je += blockDim.x) {
         int y[1];
-        half_entry<D, W, 1>(H, sT + (rev ? B - 1 - jj : jj) * P::NW, y, one);
-        if (2 * y[0] - sh == best) {
-          bn = best_h * (unsigned long long)B + (unsigned long long)jj;
-          break;
-        }
+        half_entry<D, W, 1>(H, sT + je * P::NW, y, one);
+        if (2 * y[0] - sh == best) jbest = min(jbest, rev ? B - 1 - je : je);
       }
+      jbest = block_min(jbest);
+      if (jbest != INT_MAX) bn = best_h * (unsigned long long)B + (unsigned long long)jbest;
       bv = (long long)best - pr.value_offset;   // the offset holds the value bias
     }
-    block_best(bv, bn);
     if (threadIdx.x == 0) { args.chunk_results[c].value = bv; args.chunk_results[c].index = bn; }
   }
 }

@@ -49,23 +49,6 @@ struct BatchArgs {
 constexpr int kBatchThreads = 128;
 constexpr int kBatchMaxThreads = 128;
 
-// block-wide (max value, smallest index); the result is valid in thread 0
-__device__ __forceinline__ void block_best(long long& v, unsigned long long& n) {
-  __shared__ long long s_v[32];
-  __shared__ unsigned long long s_n[32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nwarps = (blockDim.x + 31) >> 5;
-  warp_best(v, n);
-  __syncthreads();
-  if (lane == 0) { s_v[wid] = v; s_n[wid] = n; }
-  __syncthreads();
-  if (wid == 0) {
-    v = lane < nwarps ? s_v[lane] : LLONG_MIN;
-    n = lane < nwarps ? s_n[lane] : ULLONG_MAX;
-    warp_best(v, n);
-  }
-}
-
 // Table entry j (the low rows' partial sums for low labeling j, in Gray
 // order) of a D-vector problem, written to e.
 template <int D, int WB, int WA>
@@ -194,19 +177,17 @@ __global__ void __launch_bounds__(kBatchMaxThreads) batch_table_kernel(const Bat
     }
     long long bv = LLONG_MIN;
     unsigned long long bn = ULLONG_MAX;
+    block_top(best, best_h);
     if (best != INT_MIN) {
       seed_high<D, WB, WA>(H, sA, sH0, k, nh, best_h);
       const bool rev = (best_h & 1ull) != 0ull;
-      for (int jj = 0; jj < B; ++jj) {
-        const int je = rev ? B - 1 - jj : jj;
-        if (entry_value<D, WB, WA>(H, sT + je * NW) == best) {
-          bn = best_h * (unsigned long long)B + (unsigned long long)jj;
-          break;
-        }
-      }
+      int jbest = INT_MAX;
+      for (int je = threadIdx.x; je < B; je += blockDim.x)
+        if (entry_value<D, WB, WA>(H, sT + je * NW) == best) jbest = min(jbest, rev ? B - 1 - je : je);
+      jbest = block_min(jbest);
+      if (jbest != INT_MAX) bn = best_h * (unsigned long long)B + (unsigned long long)jbest;
       bv = (long long)best - pr.value_offset;
     }
-    block_best(bv, bn);
     if (threadIdx.x == 0) { args.chunk_results[c].value = bv; args.chunk_results[c].index = bn; }
   }
 }
@@ -350,41 +331,41 @@ __global__ void __launch_bounds__(kBatchMaxThreads) batch_split_kernel(const Bat
     }
     long long bv = LLONG_MIN;
     unsigned long long bn = ULLONG_MAX;
-    if (best != INT_MIN) {   // the pair holds the same best and best_h
+    block_top(best, best_h);   // the pair holds the same best and best_h
+    if (best != INT_MIN) {
       seed_high<D, WH, 0>(H, sA, sH0, k, nh, best_h);
       const bool rev = (best_h & 1ull) != 0ull;
-      for (int jj = 0; jj < B; ++jj) {
-        const int je = rev ? B - 1 - jj : jj;
+      int jbest = INT_MAX;
+      for (int je = threadIdx.x >> 1; je < B; je += blockDim.x >> 1) {
         int v = entry_value<D, WH, 0>(H, sT + je * NWH);
         v += __shfl_xor_sync(pair, v, 1);
-        if (v == best) {
-          bn = best_h * (unsigned long long)B + (unsigned long long)jj;
-          break;
-        }
+        if (v == best) jbest = min(jbest, rev ? B - 1 - je : je);
       }
+      jbest = block_min(jbest);
+      if (jbest != INT_MAX) bn = best_h * (unsigned long long)B + (unsigned long long)jbest;
       bv = (long long)best - pr.value_offset;
     }
-    block_best(bv, bn);
     if (threadIdx.x == 0) { args.chunk_results[c].value = bv; args.chunk_results[c].index = bn; }
   }
 }
 
-// Fold each matrix's chunk slots [ranges[2p], ranges[2p+1]) into results[p].
+// Fold each matrix's chunk slots [ranges[2p], ranges[2p+1]) into results[p],
+// a warp per matrix.
 // (A template so that every translation unit including this header may see
 // its definition.)
 template <int Unused = 0>
 __global__ void batch_fold_kernel(const Slot* chunk_results, const int* ranges, int nproblems,
                                   Slot* results) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (p >= nproblems) return;
   long long v = LLONG_MIN;
   unsigned long long n = ULLONG_MAX;
-  for (int c = ranges[2 * p]; c < ranges[2 * p + 1]; ++c) {
+  for (int c = ranges[2 * p] + lane; c < ranges[2 * p + 1]; c += 32) {
     const Slot s = chunk_results[c];
     if (better(s.value, s.index, v, n)) { v = s.value; n = s.index; }
   }
-  results[p].value = v;
-  results[p].index = n;
+  warp_best(v, n);
+  if (lane == 0) { results[p].value = v; results[p].index = n; }
 }
 
 }  // namespace ld

@@ -364,10 +364,12 @@ __global__ void __launch_bounds__(kTableThreads, half_min_blocks(D, W, S, K)) ha
     const unsigned long long oh = __shfl_xor_sync(gmask, best_h, off, S);
     if (ob > best || (ob == best && oh < best_h)) { best = ob; best_h = oh; }
   }
-  // the first index attaining it: rescan that block for the smallest Gray
-  // position (the low word is read backwards for odd h)
+  // the first index attaining the block's best: the smallest Gray position
+  // among the entries of its block at the maximum, a tile per group (the low
+  // word is read backwards for odd h)
   long long bv = LLONG_MIN;
   unsigned long long bn = ULLONG_MAX;
+  block_top(best, best_h);
   if (best != INT_MIN) {
     half_seed<D, W>(H[0], sA, sH0, k, nh, best_h);
     int sh = half_sh<D, W>(H[0]);
@@ -375,14 +377,13 @@ __global__ void __launch_bounds__(kTableThreads, half_min_blocks(D, W, S, K)) ha
     for (int off = 1; off < S; off <<= 1) sh += __shfl_xor_sync(gmask, sh, off, S);
     const bool rev = (best_h & 1ull) != 0ull;
     int jbest = INT_MAX;
-    for (int j0 = 0; j0 < Bp; j0 += S) {
+    for (int j0 = (int)threadIdx.x / S * S; j0 < Bp; j0 += blockDim.x) {
       int y[1];
       half_tile<D, W, S, 1>(H, sT, j0, g, gmask, src, y, one);
       const int je = j0 + g;
       if (je < B && 2 * y[0] - sh == best) jbest = min(jbest, rev ? B - 1 - je : je);
     }
-#pragma unroll
-    for (int off = 1; off < S; off <<= 1) jbest = min(jbest, __shfl_xor_sync(gmask, jbest, off, S));
+    jbest = block_min(jbest);
     if (jbest != INT_MAX) bn = best_h * (unsigned long long)B + (unsigned long long)jbest;
     bv = (long long)best + ha.value_bias - args.value_offset;
   }

@@ -267,16 +267,16 @@ __global__ void __launch_bounds__(kTableThreads) table_split_kernel(const SplitA
     const unsigned long long oh = __shfl_xor_sync(gmask, best_h, off, S);
     if (ob > best || (ob == best && oh < best_h)) { best = ob; best_h = oh; }
   }
-  // the first index attaining it: rescan that block (every lane of the
-  // group takes part), the smallest Gray position among the entries at the
-  // maximum
+  // the first index attaining the block's best: the smallest Gray position
+  // among the entries of its block at the maximum, a tile per group
   long long bv = LLONG_MIN;
   unsigned long long bn = ULLONG_MAX;
+  block_top(best, best_h);
   if (best != INT_MIN) {
     seed_high<D, SB, SA>(H, sA, sH0, k, nh, best_h);
     const int p0 = (int)(best_h & 1ull);
     int jbest = INT_MAX;
-    for (int j0 = 0; j0 < Bp; j0 += S) {
+    for (int j0 = (int)threadIdx.x / S * S; j0 < Bp; j0 += blockDim.x) {
       const int v = split_tile<D, SB, SA, S>(H, sT, j0, g, gmask, src);
       const int je = j0 + g;
       if (je < B && v == best) {
@@ -286,8 +286,7 @@ __global__ void __launch_bounds__(kTableThreads) table_split_kernel(const SplitA
         jbest = min(jbest, jj);
       }
     }
-#pragma unroll
-    for (int off = 1; off < S; off <<= 1) jbest = min(jbest, __shfl_xor_sync(gmask, jbest, off, S));
+    jbest = block_min(jbest);
     if (jbest != INT_MAX) bn = best_h * (unsigned long long)B + (unsigned long long)jbest;
     bv = (long long)best - args.value_offset;
   }

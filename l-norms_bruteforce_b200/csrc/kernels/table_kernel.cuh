@@ -728,32 +728,24 @@ __global__ void __launch_bounds__(kTableThreads, (table_min_blocks<D, PAIR>())) 
   }
   }
 
-  // The first index attaining the thread's best: rescan its block in the
-  // Gray order of the low part (reversed for odd h).
+  // The first index attaining the block's best: the smallest position among
+  // the entries of its block at that value.
   long long bv = LLONG_MIN;
   unsigned long long bn = ULLONG_MAX;
+  block_top(best, best_h);
   if (best != INT_MIN) {
     seed_high<D, WB, WA>(H, sA, sH0, k, nh, best_h);
-    if constexpr (D >= 4) {
-      // every entry once, in table order; an entry that attains the best
-      // (rare) is mapped to its block position, and the smallest is kept
-      int jbest = INT_MAX;
-      const int p0 = (int)(best_h & 1ull);
-      for (int je = 0; je < B; ++je)
-        if (entry_value<D, WB, WA, LIN>(H, sT + je * NW) == best)
-          jbest = min(jbest, block_pos_of_entry<D>(je, k, p0));
-      if (jbest != INT_MAX) bn = best_h * (unsigned long long)B + (unsigned long long)jbest;
-    } else {
-      // d <= 3: the low word is read backwards for odd h
-      const bool rev = (best_h & 1ull) != 0ull;
-      for (int jj = 0; jj < B; ++jj) {
-        const int je = rev ? B - 1 - jj : jj;
-        if (entry_value<D, WB, WA, LIN>(H, sT + je * NW) == best) {
-          bn = best_h * (unsigned long long)B + (unsigned long long)jj;
-          break;
-        }
+    const int p0 = (int)(best_h & 1ull);
+    int jbest = INT_MAX;
+    for (int je = threadIdx.x; je < B; je += blockDim.x)
+      if (entry_value<D, WB, WA, LIN>(H, sT + je * NW) == best) {
+        int jj;
+        if constexpr (D >= 4) jj = block_pos_of_entry<D>(je, k, p0);
+        else jj = p0 ? B - 1 - je : je;   // d <= 3: the low word is read backwards for odd h
+        jbest = min(jbest, jj);
       }
-    }
+    jbest = block_min(jbest);
+    if (jbest != INT_MAX) bn = best_h * (unsigned long long)B + (unsigned long long)jbest;
     bv = (long long)best - args.value_offset;
   }
   grid_reduce(bv, bn, args.red);
