@@ -50,7 +50,9 @@ typedef struct {
                               L_CUDA.cu:80 strict '>' and :347 strict '<')          */
     uint64_t labelings;    /* labelings the solve covered (evaluated, or skipped by
                               a bound or by label symmetry)                        */
-    float kernel_ms;       /* device time of the solve's launches (CUDA events)     */
+    float kernel_ms;       /* device time of the solve's launches (plans and the
+                              pruned search: CUDA events; ld_solve_reduced: the
+                              first block's start to the last one's end)           */
     int32_t kernel_kind;   /* LD_KERNEL_* actually used                             */
     int32_t lane_bits;     /* 8, 32 or 64: arithmetic lane width used (32: also two
                               columns per 32-bit word where they fit)               */

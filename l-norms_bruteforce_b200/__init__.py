@@ -395,7 +395,7 @@ class Problem:
         name = C.create_string_buffer(64)
         _check(lib().ld_problem_report(self._h, C.byref(res), strat.ctypes.data_as(_I32P), strat.size,
                                        C.byref(cnt), name, len(name)))
-        text = "".join(f"{int(v)}\n" for v in strat[: cnt.value])
+        text = "".join(f"{v}\n" for v in strat[: cnt.value].tolist())
         return name.value.decode(), text
 
 

@@ -282,7 +282,7 @@ static bool half_split_choose(const int64_t* a, int R, int C, int d, int margina
       if (o.low_rows >= 0 && k != std::min(o.low_rows, F)) continue;
       const int Bp = (int)((B + S - 1) / S * S);
       const size_t smem = (size_t)S * (ld::half_region_words(d, W, R, Bp) + 28) * sizeof(uint32_t);
-      if (smem > 227u * 1024u) break;
+      if (smem > 225u * 1024u) break;   // beside the kernel's own arrays
       double units = (double)ipow(base, F - k);
       if (d >= 3 && !o.enumerate_all && F - k > 0) {
         uint64_t pass = 0;
@@ -584,7 +584,7 @@ void ldsolve::split_range(unsigned long long n, int idx, int count, unsigned lon
 // the caller.  `shared` selects the per-device workspace instead of owned
 // resources.
 ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int marginal, const ld_options* opt,
-                            Resources* shared, ld_plan** out) {
+                            Resources* shared, ld_plan** out, bool one_shot) {
   ld_options o;
   if (opt) o = *opt; else ld_options_init(&o);
   if (!a || R < 1 || C < 1) return ld_fail(LD_ERR_ARG, "empty matrix (%d x %d)", R, C);
@@ -869,11 +869,14 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
   // scratch header: counter 0, gvalue LLONG_MIN
   const long long gmin = LLONG_MIN;
   memcpy(image.data() + kOffGvalue, &gmin, sizeof gmin);
+  const unsigned long long never = ULLONG_MAX;
+  memcpy(image.data() + kOffStart, &never, sizeof never);
 
   const size_t off_slots = align256(p->upload_bytes);
   const size_t dbytes = off_slots + align256((size_t)p->blocks * sizeof(ld::Slot));
   p->res = shared ? shared : &p->own;
-  st = resources_acquire(p->res, o.device, (cudaStream_t)o.stream, dbytes, p->upload_bytes);
+  const size_t off_host = align256(p->upload_bytes);
+  st = resources_acquire(p->res, o.device, (cudaStream_t)o.stream, dbytes, off_host + sizeof(ld::HostSlot));
   if (st != LD_OK) { plan_free(p); return st; }
   char* base_ptr = (char*)p->res->dmem;
   p->red.counter = (unsigned int*)(base_ptr + kOffCounter);
@@ -884,6 +887,11 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
   // in the upload image, reset by each launch's last block)
   p->red.work = (p->ch.kind == LD_KERNEL_TABLE && (p->ch.S == 0 || p->ch.HW > 0) && o.walk_fetch >= 0)
                     ? (unsigned long long*)(base_ptr + kOffWork) : nullptr;
+  if (one_shot) {
+    p->host = (ld::HostSlot*)((char*)p->res->hstage + off_host);
+    p->red.host = p->host;
+    p->red.start = (unsigned long long*)(base_ptr + kOffStart);
+  }
   memcpy(p->res->hstage, image.data(), p->upload_bytes);
   cudaError_t ce = cudaMemcpyAsync(p->res->dmem, p->res->hstage, p->upload_bytes, cudaMemcpyHostToDevice,
                                    p->res->stream);
@@ -898,7 +906,7 @@ ld_status ldsolve::plan_enqueue(ld_plan* p) {
   Resources* r = p->res;
   char* base_ptr = (char*)r->dmem;
   LD_CUDA(cudaSetDevice(p->device));
-  LD_CUDA(cudaEventRecord(r->ev0, r->stream));
+  if (!p->host) LD_CUDA(cudaEventRecord(r->ev0, r->stream));
   if (p->ch.kind == LD_KERNEL_TABLE) {
     ld::TableArgs args;
     args.A = (const uint32_t*)(base_ptr + p->off_A);
@@ -982,7 +990,7 @@ ld_status ldsolve::plan_enqueue(ld_plan* p) {
     void* params[] = {&args};
     LD_CUDA(cudaLaunchKernel(p->kfn, dim3(p->blocks), dim3(p->tpb), params, 0, r->stream));
   }
-  LD_CUDA(cudaEventRecord(r->ev1, r->stream));
+  if (!p->host) LD_CUDA(cudaEventRecord(r->ev1, r->stream));
   p->launched = true;
   return LD_OK;
 }
@@ -999,16 +1007,24 @@ ld_status ldsolve::plan_fetch(ld_plan* p, ld_result* res, int32_t* strategy) {
   if (!p->launched) return ld_fail(LD_ERR_ARG, "plan has not been launched");
   Resources* r = p->res;
   LD_CUDA(cudaSetDevice(p->device));
-  ld::Slot* h = (ld::Slot*)((char*)r->hstage + kOffResult);
-  LD_CUDA(cudaMemcpyAsync(h, p->red.result, sizeof(ld::Slot), cudaMemcpyDeviceToHost, r->stream));
-  LD_CUDA(cudaStreamSynchronize(r->stream));
+  ld::Slot h;
   float ms = 0.f;
-  LD_CUDA(cudaEventElapsedTime(&ms, r->ev0, r->ev1));
-  if (p->ch.kind == LD_KERNEL_TABLE && p->ch.tc && h->value == LLONG_MAX)
+  if (p->host) {
+    LD_CUDA(cudaStreamSynchronize(r->stream));
+    h = ld::Slot{p->host->value, p->host->index};
+    ms = (float)(p->host->t1 - p->host->t0) * 1e-6f;
+  } else {
+    ld::Slot* copy = (ld::Slot*)((char*)r->hstage + kOffResult);
+    LD_CUDA(cudaMemcpyAsync(copy, p->red.result, sizeof(ld::Slot), cudaMemcpyDeviceToHost, r->stream));
+    LD_CUDA(cudaStreamSynchronize(r->stream));
+    LD_CUDA(cudaEventElapsedTime(&ms, r->ev0, r->ev1));
+    h = *copy;
+  }
+  if (p->ch.kind == LD_KERNEL_TABLE && p->ch.tc && h.value == LLONG_MAX)
     return ld_fail(LD_ERR_TIMEOUT, "tensor-core enumeration: a device-side wait ran out");
   memset(res, 0, sizeof *res);
-  res->value = h->value;
-  res->gray_index = h->index;
+  res->value = h.value;
+  res->gray_index = h.index;
   res->labelings = p->ch.kind == LD_KERNEL_TABLE
                        ? (p->walk_end - p->walk_begin) * p->walk_len * (unsigned long long)p->B
                        : p->n_end - p->n_begin;
@@ -1016,7 +1032,7 @@ ld_status ldsolve::plan_fetch(ld_plan* p, ld_result* res, int32_t* strategy) {
   res->kernel_kind = p->ch.kind;
   res->lane_bits = p->ch.lane_bits;
   res->h2d_bytes = p->uploaded ? p->upload_bytes : 0;
-  res->d2h_bytes = sizeof(ld::Slot);
+  res->d2h_bytes = p->host ? sizeof(ld::HostSlot) : sizeof(ld::Slot);
   res->evaluated = plan_evaluated(p);
   if (strategy) ld_gray_labels(res->gray_index, p->R, p->d, strategy);
   p->uploaded = false;
@@ -1092,7 +1108,7 @@ extern "C" ld_status ld_solve_reduced(const int64_t* a, int32_t rows, int32_t co
   std::unique_lock<std::mutex> lk(g_ws_mu[dev], std::defer_lock);
   if (use_ws) lk.lock();
   ld_plan* p = nullptr;
-  ld_status st = plan_build(a, rows, cols, d, marginal, opt, use_ws ? &g_ws[dev] : nullptr, &p);
+  ld_status st = plan_build(a, rows, cols, d, marginal, opt, use_ws ? &g_ws[dev] : nullptr, &p, true);
   if (st != LD_OK) return st;
   st = plan_enqueue(p);
   if (st == LD_OK) st = plan_fetch(p, res, strategy);

@@ -98,7 +98,7 @@ extern Resources g_pws[64];
 
 // a plan's device image: reduction header, then totals, initial H, table
 // bias and packed rows
-constexpr size_t kOffCounter = 0, kOffGvalue = 8, kOffResult = 16, kOffWork = 32;
+constexpr size_t kOffCounter = 0, kOffGvalue = 8, kOffResult = 16, kOffWork = 32, kOffStart = 40;
 constexpr size_t kOffTot = 256, kOffH0 = 512, kOffTb = 768, kOffA = 1024;
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -137,15 +137,19 @@ struct ld_plan {
   ld::Reduce red{};
   const void* kfn = nullptr;
   bool launched = false;
+  ld::HostSlot* host = nullptr;   // one-shot: the result in pinned host memory
 };
 
 namespace ldsolve {
 
 void plan_free(ld_plan* p);
 // geometry, kernel choice and the upload image; `shared` selects a
-// per-device workspace instead of the plan's own resources
+// per-device workspace instead of the plan's own resources.  one_shot: the
+// plan is launched and fetched once by the same call, so the kernel writes its
+// result and times to pinned host memory (else the result is copied from the
+// plan's device slot, which the caller may combine with other ranks' first)
 ld_status plan_build(const int64_t* a, int R, int C, int d, int marginal, const ld_options* opt,
-                     Resources* shared, ld_plan** out);
+                     Resources* shared, ld_plan** out, bool one_shot = false);
 ld_status plan_enqueue(ld_plan* p);
 unsigned long long plan_evaluated(const ld_plan* p);
 ld_status plan_fetch(ld_plan* p, ld_result* res, int32_t* strategy);

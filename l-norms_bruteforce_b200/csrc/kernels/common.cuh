@@ -15,6 +15,14 @@ struct Slot {
   unsigned long long index; // its Gray index (ULLONG_MAX = none)
 };
 
+// The result of a one-shot solve in pinned host memory, written by the kernel:
+// a copy queued behind a small kernel took 8 us, a pair of timing events 6.
+struct HostSlot {
+  long long value;
+  unsigned long long index;
+  unsigned long long t0, t1;   // ns: the first block's start, the last one's end
+};
+
 // Scratch a launch reduces through.  `slots` holds one entry per block;
 // `counter` and `gvalue` must be 0 / LLONG_MIN before the first launch and
 // are restored by the last block of every launch.
@@ -25,7 +33,26 @@ struct Reduce {
   Slot* result;
   unsigned long long* work;   // walk counter the launch's warps fetch from (0 before
                               // the launch, reset by the last block), or null
+  HostSlot* host = nullptr;   // also write the result here
+  unsigned long long* start = nullptr;   // with host: ULLONG_MAX before the launch, re-armed likewise
 };
+
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// The block's start time, kept by thread 0 for grid_reduce.
+__device__ __forceinline__ unsigned long long& block_clock() {
+  __shared__ unsigned long long t;
+  return t;
+}
+
+// First thing in a kernel that may reduce into a HostSlot.
+__device__ __forceinline__ void block_start() {
+  if (threadIdx.x == 0) block_clock() = global_ns();
+}
 
 // ---- packed integer lanes ----------------------------------------------
 // PK columns share one 32-bit word as independent signed lanes of 32/PK
@@ -126,6 +153,7 @@ __device__ __forceinline__ bool grid_reduce(long long v, unsigned long long n, c
       R.slots[blockIdx.x].value = v;
       R.slots[blockIdx.x].index = n;
       if (v != LLONG_MIN) atomicMax(R.gvalue, v);
+      if (R.host) atomicMin(R.start, block_clock());
       __threadfence();
       unsigned int done = atomicAdd(R.counter, 1u);
       s_last = (done == gridDim.x - 1);
@@ -151,6 +179,9 @@ __device__ __forceinline__ bool grid_reduce(long long v, unsigned long long n, c
     for (int w = 0; w < nwarps; ++w) if (s_n[w] < best) best = s_n[w];
     R.result->value = gmax;
     R.result->index = best;
+    if (R.host) {
+      *R.host = HostSlot{gmax, best, atomicExch(R.start, ULLONG_MAX), global_ns()};
+    }
     *R.gvalue = LLONG_MIN;
     *R.counter = 0u;
     if (R.work) *R.work = 0ull;   // every block has finished fetching walks

@@ -270,6 +270,7 @@ __global__ void __launch_bounds__(kTableThreads, half_min_blocks(D, W, S, K)) ha
   static_assert(D >= 1 && D <= 3 && (S == 1 || S == 2 || S == 4 || S == 8) && (K == 1 || K == 2), "");
   const TableArgs& args = ha.t;
   extern __shared__ __align__(16) uint32_t smem[];
+  block_start();
   const int R = args.R, k = args.k, B = args.B, Bp = ha.Bp, span = ha.span;
   const uint32_t one = ha.one;
   const int nh = R - 1 - k;

@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(kTableThreads) table_split_kernel(const SplitA
   constexpr int NW = Sh::NW;     // words of a slice entry (D * PW)
   const TableArgs& args = sa.t;
   extern __shared__ __align__(16) uint32_t smem[];
+  block_start();
   const int R = args.R, k = args.k, B = args.B, Bp = sa.Bp, W = sa.W, span = sa.span;
   const int nh = R - 1 - k;
   const int head = (R * PW + 3 * PW + 3) & ~3;

@@ -556,6 +556,7 @@ __global__ void __launch_bounds__(kTableThreads, (table_min_blocks<D, PAIR>())) 
   using S = Shape<D, WB, WA>;
   constexpr int WT = S::WT, WV = S::WV, NW = S::NW;
   extern __shared__ __align__(16) uint32_t smem[];
+  block_start();
   const int R = args.R, k = args.k, B = args.B;
   const int nh = R - 1 - k;  // high rows
   uint32_t* sA = smem;

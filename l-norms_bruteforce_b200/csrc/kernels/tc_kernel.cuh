@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
   constexpr int kCS = tc_chunk_steps(kSteps), kChunks = (kSteps + kCS - 1) / kCS;
   constexpr int kSets = 2, kThreads = kTcThreads;
   extern __shared__ __align__(1024) unsigned char tc_mem[];
+  block_start();
   // Per set: two chunks, one accumulator buffer, and four slots for the bases
   // of its tiles (their four partial sums per row) and its walks.  A slot is
   // written when the tile's first chunk is taken: then the products of the
@@ -630,7 +631,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
     }
   }
   __syncthreads();
-  if (tid == 0) a.red.result->index = gh * (unsigned long long)a.B + (unsigned long long)s_first;
+  if (tid == 0) {
+    const unsigned long long n = gh * (unsigned long long)a.B + (unsigned long long)s_first;
+    a.red.result->index = n;
+    if (a.red.host) { a.red.host->index = n; a.red.host->t1 = global_ns(); }
+  }
 }
 
 }  // namespace ld

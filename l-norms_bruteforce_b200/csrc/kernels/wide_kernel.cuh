@@ -202,6 +202,7 @@ static __device__ __forceinline__ unsigned long long walk_of_rank_rt(unsigned lo
 
 template <typename IT, int PC, bool MULTI, bool SYM = false>
 __global__ void __launch_bounds__(kWideThreads) wide_kernel(const WideArgs<IT> args) {
+  block_start();
   const int lane = threadIdx.x & 31;
   const unsigned long long gw = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
