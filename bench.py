@@ -108,9 +108,14 @@ def issue_ops_per_labeling(desc: str, d: int, cols: int) -> tuple[int, str]:
     vector (D vectors per labeling: 1 for L_1/LM, 2 or 3 for d = 2, 3); both
     issue at half the ALU pipe's add/xor rate, so each costs 2 slots of the
     int32 add/xor peak.  The LM instances that add the marginal column
-    linearly skip its word.  Wide kernel: the plain count."""
+    linearly skip its word.  Wide kernel: the plain count.  Tensor-core form
+    (tc=): int8 tensor operations instead, against INT8_PEAK."""
     f = dict(kv.split("=") for kv in desc.replace("int32 words", "int32_words")
              .replace("int8x4 words", "int8x4_words").split() if "=" in kv)
+    if int(f.get("tc", 0)) > 0:
+        # tensor-core form: a 0/1 feature of the high index times a weight of
+        # the low one, two operations each
+        return 2 * int(f["tc"]), f"2 x {f['tc']} feature products on the tensor cores (u8 x s8)"
     if desc.startswith("table") and "int32_words" in f:
         D, wb, wa = int(f["D"]), int(f["int32_words"]), int(f["int8x4_words"])
         if int(f.get("half", 0)) > 0:
@@ -130,11 +135,15 @@ def issue_ops_per_labeling(desc: str, d: int, cols: int) -> tuple[int, str]:
     return ops_per_labeling(d, cols), "plain count (wide kernel)"
 
 
-# DRAM traffic of one launch of the config-2 table kernel, from the ncu
-# capture summarised in profiles/table_kernel_config2_LM_34x37.md
-# (dram__bytes_read.sum + dram__bytes_write.sum); the kernel is ALU-bound and
-# reads only its matrix image.
-TRAFFIC_BYTES = {2: 62208}
+# int8 tensor operations per second: products of 128 x 256 x 32 issued back to
+# back from tensor memory, 7800 multiply-adds per clock and SM (measured; 148
+# SMs at 1965 MHz).
+INT8_PEAK = 2 * 7800 * 148 * 1.965e9
+
+# DRAM traffic of one launch of the kernel that solves config 2, from the ncu
+# capture summarised in profiles/tc_kernel.md (dram__bytes_read.sum +
+# dram__bytes_write.sum); it reads only its matrix image.
+TRAFFIC_BYTES = {2: 94464}
 
 
 # ---------------------------------------------------------------- clocks
@@ -582,7 +591,8 @@ def run_ours(args) -> None:
         desc = plan.describe()
         opl = ops_per_labeling(d, info["cols"])
         iopl, iwhat = issue_ops_per_labeling(desc, d, info["cols"])
-        peak_ops, _ = ld.int32_peak(local)
+        tensor = " tc=" in desc and not desc.endswith(" tc=0")
+        peak_ops = INT8_PEAK if tensor else ld.int32_peak(local)[0]
         # labelings the kernel computed a value for (d >= 3: the walks that
         # hold no smallest index of a label-permutation class are skipped)
         evaluated = int(sol.evaluated)
@@ -600,15 +610,16 @@ def run_ours(args) -> None:
                                            f"1..{d - 1} are skipped") if d >= 3 and evaluated < hi - lo else None,
                         "parallelism": f"gray-index shards x{world}" if world > 1 else "single GPU",
                         "kernel": desc, "value": sol.value, "gray_index": sol.gray_index},
-            "roofline": {"bound": "int32", "achieved": achieved / 1e12, "peak": peak_ops / 1e12,
-                         "unit": "Tops/s", "frac": achieved / peak_ops,
+            "roofline": {"bound": "tensor int8" if tensor else "int32", "achieved": achieved / 1e12,
+                         "peak": peak_ops / 1e12, "unit": "Tops/s", "frac": achieved / peak_ops,
                          "traffic": TRAFFIC_BYTES.get(args.config) if world == 1 and not args.wide else None,
                          "ops_per_labeling": iopl,
                          "plain_method": {"ops_per_labeling": opl, "achieved": opl * rate / 1e12,
                                           "x_peak": opl * rate / peak_ops},
-                         "note": f"achieved = {iopl} int32 issue slots per labeling ({iwhat}) x evaluated "
-                                 f"labelings/s; "
-                                 f"peak = int32 add/xor microbenchmark measured in this run; plain_method "
+                         "note": f"achieved = {iopl} {'int8 tensor operations' if tensor else 'int32 issue slots'} "
+                                 f"per labeling ({iwhat}) x evaluated labelings/s; "
+                                 f"peak = {'128x256x32 products issued back to back, measured' if tensor else 'int32 add/xor microbenchmark measured in this run'}"
+                                 f"; plain_method "
                                  f"counts the {'3m' if d == 1 else '6m'} ops the plain enumeration spends per "
                                  f"labeling (m={info['cols']}), which the table decomposition avoids"},
             "e2e": {"value": e2e_value, "unit": "labelings/s", "h2d_bytes_per_step": h2d,
