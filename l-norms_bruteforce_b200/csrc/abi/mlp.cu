@@ -31,7 +31,7 @@ size_t gemm_smem() {
   // Each CTA holds BN of the SM's 512 TMEM columns; the shared-memory request
   // is raised so that no more CTAs share an SM than TMEM can hold at once
   // (233472 bytes of shared memory per SM, 1 KB reserved per CTA).
-  const size_t tiles = 2 * ((size_t)ld::mlp::kTileM * ld::mlp::kTileK * 2 + (size_t)BN * ld::mlp::kTileK * 2);
+  const size_t tiles = ld::mlp::gemm_stages(BN) * ((size_t)ld::mlp::kTileM * ld::mlp::kTileK * 2 + (size_t)BN * ld::mlp::kTileK * 2);
   const size_t cap = 233472 / (512 / BN + 1) + 1024;
   return tiles > cap ? tiles : cap;
 }
@@ -53,13 +53,15 @@ cudaError_t gemm_init() {
 template <int BN>
 cudaError_t launch_gemm(const ld::mlp::GemmArgs& g, cudaStream_t s) {
   dim3 grid(g.M / ld::mlp::kTileM, g.N / BN);
-  ld::mlp::tc_gemm_kernel<BN><<<grid, 128, gemm_smem<BN>(), s>>>(g);
+  ld::mlp::GemmGroup group{};
+  group.g[0] = g;
+  ld::mlp::tc_gemm_kernel<BN><<<grid, 128, gemm_smem<BN>(), s>>>(group);
   return cudaGetLastError();
 }
 
 cudaError_t gemm(const bf16* A, const bf16* B, int M, int N, int K, float* C, bf16* H, bf16* HT,
-                 const float* bias, int relu, int* err, cudaStream_t s) {
-  ld::mlp::GemmArgs g{A, B, M, N, K, C, H, HT, bias, relu, err};
+                 const float* bias, int relu, int* err, cudaStream_t s, const bf16* gate = nullptr) {
+  ld::mlp::GemmArgs g{A, B, M, N, K, C, H, HT, bias, relu, err, gate};
   // these GEMMs are small: prefer the tile width that gives the most CTAs
   // while a wider tile still fills the 148 SMs
   const int tiles_m = M / ld::mlp::kTileM;
@@ -84,13 +86,13 @@ struct ld_mlp {
   // bf16 operands
   bf16 *W1b, *W2b, *W2T, *W3b, *W3T;
   bf16 *Xb, *XT, *H1, *H1T, *H2, *H2T, *dZ3, *dZ3T, *dZ2, *dZ2T, *dZ1T;
-  float *Xf, *Z3, *Tt, *Mk, *dH2, *dH1, *loss, *hp;
+  float *Xf, *Z3, *Tt, *Mk, *loss, *hp;
   int* err;
   int step = 0;
   // pinned staging: inputs (x, targets, mask, step parameters) and results
   // (logits, loss, error flag); the graphs copy from and to these
   void* hmem = nullptr;
-  float *hX, *hT, *hM, *hHp, *hZ, *hLoss;
+  float *hX, *hT, *hM, *hHp, *hZ, *hLoss, *hG;
   int* hErr;
   // captured CUDA graphs: one training step, one forward pass
   cudaGraphExec_t train_exec = nullptr, fwd_exec = nullptr;
@@ -178,19 +180,20 @@ cudaError_t enqueue_backward(ld_mlp* n) {
                                                                      n->skip != 0.f ? n->Xf : nullptr, n->skip,
                                                                      n->dZ3, n->dZ3T, n->loss);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  // W3: [kOutGP x B] x [kHid x B]^T (rows kOutP.. of dZ3T are zero)
-  if ((e = gemm(n->dZ3T, n->H2T, kOutGP, kHid, B, n->gW3, nullptr, nullptr, nullptr, 0, n->err, n->s)) != cudaSuccess) return e;
-  if ((e = gemm(n->dZ3, n->W3T, B, kHid, kOutP, n->dH2, nullptr, nullptr, nullptr, 0, n->err, n->s)) != cudaSuccess) return e;
-  ld::mlp::relu_grad_kernel<<<blocks_for(B * kHid), 256, 0, n->s>>>(n->dH2, n->H2, B, kHid, n->dZ2, n->dZ2T);
+  // dZ2 = (dZ3 W3) where H2 > 0, then dZ1: the ReLU's derivative in the epilogue
+  if ((e = gemm(n->dZ3, n->W3T, B, kHid, kOutP, nullptr, n->dZ2, n->dZ2T, nullptr, 0, n->err, n->s, n->H2)) != cudaSuccess) return e;
+  if ((e = gemm(n->dZ2, n->W2T, B, kHid, kHid, nullptr, nullptr, n->dZ1T, nullptr, 0, n->err, n->s, n->H1)) != cudaSuccess) return e;
+  // the weight gradients in one launch; W3: [kOutGP x B] x [kHid x B]^T (rows
+  // kOutP.. of dZ3T are zero)
+  ld::mlp::GemmGroup w{};
+  w.g[0] = ld::mlp::GemmArgs{n->dZ3T, n->H2T, kOutGP, kHid, B, n->gW3, nullptr, nullptr, nullptr, 0, n->err, nullptr};
+  w.g[1] = ld::mlp::GemmArgs{n->dZ2T, n->H1T, kHid, kHid, B, n->gW2, nullptr, nullptr, nullptr, 0, n->err, nullptr};
+  w.g[2] = ld::mlp::GemmArgs{n->dZ1T, n->XT, kHid, kInP, B, n->gW1, nullptr, nullptr, nullptr, 0, n->err, nullptr};
+  const dim3 grid(kHid / ld::mlp::kTileM, kHid / 64, 3);
+  ld::mlp::tc_gemm_kernel<64><<<grid, 128, gemm_smem<64>(), n->s>>>(w);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = gemm(n->dZ2T, n->H1T, kHid, kHid, B, n->gW2, nullptr, nullptr, nullptr, 0, n->err, n->s)) != cudaSuccess) return e;
-  if ((e = gemm(n->dZ2, n->W2T, B, kHid, kHid, n->dH1, nullptr, nullptr, nullptr, 0, n->err, n->s)) != cudaSuccess) return e;
-  ld::mlp::relu_grad_kernel<<<blocks_for(B * kHid), 256, 0, n->s>>>(n->dH1, n->H1, B, kHid, nullptr, n->dZ1T);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = gemm(n->dZ1T, n->XT, kHid, kInP, B, n->gW1, nullptr, nullptr, nullptr, 0, n->err, n->s)) != cudaSuccess) return e;
-  ld::mlp::bias_grad_kernel<<<kHid / 4, 128, 0, n->s>>>(n->dZ1T, kHid, B, n->gb1);
-  ld::mlp::bias_grad_kernel<<<kHid / 4, 128, 0, n->s>>>(n->dZ2T, kHid, B, n->gb2);
-  ld::mlp::bias_grad_kernel<<<kOutP / 4, 128, 0, n->s>>>(n->dZ3T, kOutP, B, n->gb3);
+  const ld::mlp::BiasGrads bias{{n->dZ1T, n->dZ2T, n->dZ3T}, {n->gb1, n->gb2, n->gb3}, {kHid, kHid, kOutP}};
+  ld::mlp::bias_grad_kernel<<<(2 * kHid + kOutP) / 4, 128, 0, n->s>>>(bias, B);
   return cudaGetLastError();
 }
 
@@ -265,10 +268,11 @@ extern "C" ld_status ld_mlp_create(int32_t batch, uint64_t seed, float skip, int
   for (int i = 0; i < 6; ++i) {
     const size_t c = (size_t)kShapes[i].rows * kShapes[i].cols;
     f32(params_of(n, i), c);
-    f32(grads_of(n, i), i == 4 ? (size_t)kOutGP * kHid : c);
     f32(&n->m[i], c);
     f32(&n->v[i], c);
   }
+  // the gradients one after another: they come back in one copy
+  for (int i = 0; i < 6; ++i) f32(grads_of(n, i), i == 4 ? (size_t)kOutGP * kHid : (size_t)kShapes[i].rows * kShapes[i].cols);
   b16(&n->W1b, (size_t)kHid * kInP); b16(&n->W2b, (size_t)kHid * kHid); b16(&n->W2T, (size_t)kHid * kHid);
   b16(&n->W3b, (size_t)kOutP * kHid); b16(&n->W3T, (size_t)kHid * kOutP);
   b16(&n->Xb, (size_t)B * kInP); b16(&n->XT, (size_t)kInP * B);
@@ -277,7 +281,7 @@ extern "C" ld_status ld_mlp_create(int32_t batch, uint64_t seed, float skip, int
   b16(&n->dZ3, (size_t)B * kOutP); b16(&n->dZ3T, (size_t)kOutGP * B);
   b16(&n->dZ2, (size_t)B * kHid); b16(&n->dZ2T, (size_t)kHid * B); b16(&n->dZ1T, (size_t)kHid * B);
   f32(&n->Xf, (size_t)B * kInP); f32(&n->Z3, (size_t)B * kOutP); f32(&n->Tt, (size_t)B * kOutP);
-  f32(&n->Mk, (size_t)B * kOutP); f32(&n->dH2, (size_t)B * kHid); f32(&n->dH1, (size_t)B * kHid);
+  f32(&n->Mk, (size_t)B * kOutP);
   f32(&n->loss, 1);
   f32(&n->hp, ld::mlp::kHpWords);
   pieces.push_back({(void**)&n->err, 4});
@@ -307,15 +311,17 @@ extern "C" ld_status ld_mlp_create(int32_t batch, uint64_t seed, float skip, int
     return ld_fail(LD_ERR_CUDA, "network initialisation failed");
   }
   // pinned staging: x, targets, mask (batch x 64 each), logits (batch x 64),
-  // step parameters, loss, error flag
+  // step parameters, loss, error flag; gradients
   const size_t slab = sizeof(float) * (size_t)B * 64;
-  if (cudaMallocHost(&n->hmem, 4 * slab + 256) != cudaSuccess) {
+  const size_t grads = (size_t)((char*)(n->gb3 + kOutP) - (char*)n->gW1);
+  if (cudaMallocHost(&n->hmem, 4 * slab + 256 + grads) != cudaSuccess) {
     ld_mlp_destroy(n);
     return ld_fail(LD_ERR_CUDA, "pinned staging allocation failed");
   }
   char* h = (char*)n->hmem;
   n->hX = (float*)h; n->hT = (float*)(h + slab); n->hM = (float*)(h + 2 * slab); n->hZ = (float*)(h + 3 * slab);
   n->hHp = (float*)(h + 4 * slab); n->hLoss = (float*)(h + 4 * slab + 64); n->hErr = (int*)(h + 4 * slab + 128);
+  n->hG = (float*)(h + 4 * slab + 256);
   memset(n->hmem, 0, 4 * slab + 256);
   // one training step and one forward pass as CUDA graphs over fixed buffers
   ld_status st = capture(n, [&] {
@@ -417,6 +423,8 @@ extern "C" ld_status ld_mlp_gradients(ld_mlp* n, const float* x, const float* t,
   MLP_CUDA(enqueue_forward(n));
   MLP_CUDA(enqueue_backward(n));
   MLP_CUDA(enqueue_results(n, false));
+  if (grads)
+    MLP_CUDA(cudaMemcpyAsync(n->hG, n->gW1, (size_t)((char*)(n->gb3 + kOutP) - (char*)n->gW1), cudaMemcpyDeviceToHost, n->s));
   ld_status st = finish(n);
   if (st != LD_OK) return st;
   if (loss) *loss = *n->hLoss;
@@ -424,11 +432,9 @@ extern "C" ld_status ld_mlp_gradients(ld_mlp* n, const float* x, const float* t,
     float* dst = grads;
     for (int i = 0; i < 6; ++i) {
       const PShape& sh = kShapes[i];
-      const int drows = i == 4 ? kOutGP : sh.rows;
-      std::vector<float> g((size_t)drows * sh.cols);
-      MLP_CUDA(cudaMemcpy(g.data(), *grads_of(n, i), sizeof(float) * g.size(), cudaMemcpyDeviceToHost));
-      for (int r = 0; r < sh.hrows; ++r)
-        for (int c = 0; c < sh.hcols; ++c) *dst++ = g[(size_t)r * sh.cols + c];
+      const float* g = n->hG + (*grads_of(n, i) - n->gW1);
+      for (int r = 0; r < sh.hrows; ++r, dst += sh.hcols)
+        memcpy(dst, g + (size_t)r * sh.cols, sizeof(float) * sh.hcols);
     }
   }
   return LD_OK;

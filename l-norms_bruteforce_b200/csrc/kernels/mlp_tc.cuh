@@ -4,15 +4,15 @@
 //   C[M x N] = A[M x K] * B[N x K]^T      (A, B bf16, K-major; fp32 accumulate)
 //
 // One CTA (4 warps) computes a 128 x BN tile.  Per 64-wide K chunk the CTA
-// copies the A and B tiles (cp.async, two stages) into shared memory in the
+// copies the A and B tiles (cp.async, kGemmStages stages) into shared memory in the
 // canonical K-major layout without swizzle (8-row x 16-byte core matrices;
 // core matrices 128 B apart along K, 1024 B apart along M/N), one elected
 // thread issues four tcgen05.mma (K = 16 each) into a TMEM accumulator of
 // 128 lanes x BN fp32 columns and commits them to the stage's mbarrier,
 // which the CTA waits on before refilling that stage.  The epilogue reads the accumulator with
 // tcgen05.ld (warp w owns lanes 32w..32w+31, i.e. rows 32w..32w+31 of the
-// tile), optionally adds a bias and applies ReLU, and stores fp32 and/or
-// bf16 (row-major and transposed) outputs.
+// tile), optionally adds a bias and applies ReLU or a ReLU's derivative, and
+// stores fp32 and/or bf16 (row-major and transposed) outputs.
 //
 // Every wait is bounded: a wait that runs out sets *err and the CTA stops
 // issuing work; the host checks *err after the launch.
@@ -75,7 +75,19 @@ struct GemmArgs {
   const float* bias;        // N, or null
   int relu;
   int* err;
+  const __nv_bfloat16* gate;   // M x N: results where it is not positive become 0, or null
 };
+
+// Up to three products in one launch (blockIdx.z): the weight gradients, which
+// are 4, 8 and 2 tiles of 128 x 64 with all of the batch to add up (three
+// launches of 22 us each, one of 20).
+struct GemmGroup { GemmArgs g[3]; };
+
+// Stages: these products are short chains of chunks on few SMs (of 20 us for
+// K = 1024, 9 are there for a single chunk too).  Four 64-wide stages instead
+// of two: 0.9 -> 0.7 us per chunk; the wider tiles fill the SMs and keep two
+// CTAs per SM.
+constexpr int gemm_stages(int BN) { return BN == 64 ? 4 : 2; }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
@@ -84,16 +96,19 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
 
-// Two-stage pipeline: while the tensor core multiplies chunk kc out of one
-// shared-memory stage, the CTA's threads copy chunk kc + 1 into the other
-// with cp.async.  A stage is refilled only after the mbarrier of the MMAs
-// that read it has completed.
+// Pipeline: while the tensor core multiplies chunk kc out of one shared-memory
+// stage, the CTA's threads copy the next chunks into the others with cp.async.
+// A stage is refilled only after the mbarrier of the MMAs that read it has
+// completed.
 template <int BN>
-__global__ void __launch_bounds__(128) tc_gemm_kernel(const GemmArgs g) {
+__global__ void __launch_bounds__(128) tc_gemm_kernel(const GemmGroup group) {
+  const GemmArgs& g = group.g[blockIdx.z];
+  if ((int)blockIdx.x * kTileM >= g.M || (int)blockIdx.y * BN >= g.N) return;   // outside this product
+  constexpr int kStages = gemm_stages(BN);
   static_assert(BN == 64 || BN == 128 || BN == 256, "tile width");
   constexpr int kStageA = kTileM * kTileK * 2, kStageB = BN * kTileK * 2;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t mbar[2];
+  __shared__ __align__(8) uint64_t mbar[kStages];
   __shared__ uint32_t tmem_base;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.x * kTileM, n0 = blockIdx.y * BN;
@@ -107,8 +122,9 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(const GemmArgs g) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&mbar[0])), "r"(1));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&mbar[1])), "r"(1));
+#pragma unroll
+    for (int i = 0; i < kStages; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&mbar[i])), "r"(1));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -136,18 +152,16 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(const GemmArgs g) {
 
   const int nk = g.K / kTileK;
   bool ok = true;
-  load(0, 0);
+  bool good = true;
+  // one group of copies per chunk (empty past the last), kStages - 1 ahead
+#pragma unroll
+  for (int p = 0; p < kStages - 1; ++p) {
+    if (p < nk) load(p, p);
+    else cp_async_commit();
+  }
   for (int kc = 0; kc < nk; ++kc) {
-    const int st = kc & 1;
-    bool good = true;
-    if (kc + 1 < nk) {
-      // stage st ^ 1 was read by the MMAs of chunk kc - 1 (its ((kc-1)/2)-th use)
-      if (kc >= 1) good = mbar_wait(smem_u32(&mbar[st ^ 1]), (uint32_t)((kc - 1) >> 1) & 1u);
-      if (good) load(kc + 1, st ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+    const int st = kc % kStages;
+    cp_async_wait<kStages - 2>();
     // generic-proxy shared-memory writes -> visible to the tensor core
     asm volatile("fence.proxy.async.shared::cta;");
     if (__syncthreads_or(!good)) { ok = false; break; }
@@ -167,10 +181,19 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(const GemmArgs g) {
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                    :: "r"(smem_u32(&mbar[st])));
     }
+    const int next = kc + kStages - 1, into = next % kStages;
+    if (next < nk) {
+      // the stage was read by the MMAs of chunk kc - 1
+      if (kc >= 1) good = mbar_wait(smem_u32(&mbar[into]), (uint32_t)((kc - 1) / kStages) & 1u);
+      if (good) load(next, into);
+      else cp_async_commit();
+    } else {
+      cp_async_commit();
+    }
   }
   if (ok) {
     // the last commit tracks every MMA issued before it
-    const bool done = mbar_wait(smem_u32(&mbar[(nk - 1) & 1]), (uint32_t)((nk - 1) >> 1) & 1u);
+    const bool done = mbar_wait(smem_u32(&mbar[(nk - 1) % kStages]), (uint32_t)((nk - 1) / kStages) & 1u);
     ok = !__syncthreads_or(!done);
   } else {
     cp_async_wait<0>();
@@ -197,6 +220,20 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(const GemmArgs g) {
         v[j] = __uint_as_float(r[j]);
         if (g.bias) v[j] += g.bias[n0 + c0 + j];
         if (g.relu) v[j] = fmaxf(v[j], 0.f);
+      }
+      if (g.gate) {
+        const uint4* gt = reinterpret_cast<const uint4*>(g.gate + (size_t)row * g.N + n0 + c0);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const uint4 x = gt[q];
+          const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162*>(&xs[j]);
+            if (!(__low2float(b) > 0.f)) v[8 * q + 2 * j] = 0.f;
+            if (!(__high2float(b) > 0.f)) v[8 * q + 2 * j + 1] = 0.f;
+          }
+        }
       }
       if (g.C) {
         float4* dst = reinterpret_cast<float4*>(g.C + (size_t)row * g.N + n0 + c0);
@@ -255,26 +292,18 @@ __global__ void bce_grad_kernel(const float* z, const float* t, const float* mas
   if ((threadIdx.x & 31) == 0 && l != 0.f) atomicAdd(loss, l);
 }
 
-// dz = dh * (h > 0), bf16 row-major and / or transposed
-__global__ void relu_grad_kernel(const float* dh, const __nv_bfloat16* h, int rows, int cols,
-                                 __nv_bfloat16* dz, __nv_bfloat16* dzT) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * cols) return;
-  const int r = i / cols, c = i % cols;
-  const float g = __bfloat162float(h[i]) > 0.f ? dh[i] : 0.f;
-  if (dz) dz[i] = __float2bfloat16_rn(g);
-  if (dzT) dzT[(size_t)c * rows + r] = __float2bfloat16_rn(g);
-}
-
-// db[c] = sum over r of dzT[c][r] (bf16), one warp per output
-__global__ void bias_grad_kernel(const __nv_bfloat16* dzT, int cols, int rows, float* db) {
-  const int c = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+// db[c] = sum over r of dzT[c][r] (bf16) of the three layers, one warp per
+// output, in one launch
+struct BiasGrads { const __nv_bfloat16* dzT[3]; float* db[3]; int cols[3]; };
+__global__ void bias_grad_kernel(const BiasGrads a, int rows) {
+  int c = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), i = 0;
+  while (i < 3 && c >= a.cols[i]) c -= a.cols[i++];
+  if (i == 3) return;
   const int lane = threadIdx.x & 31;
-  if (c >= cols) return;
   float s = 0.f;
-  for (int r = lane; r < rows; r += 32) s += __bfloat162float(dzT[(size_t)c * rows + r]);
+  for (int r = lane; r < rows; r += 32) s += __bfloat162float(a.dzT[i][(size_t)c * rows + r]);
   for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) db[c] = s;
+  if (lane == 0) a.db[i][c] = s;
 }
 
 // Adam on fp32 master weights w (rows x cols, gradient g); refreshes the
