@@ -261,7 +261,8 @@ static bool half_allowed(int d, const ld_options& o) { return d <= 3 && o.lane_b
 // entry and lane are 2.5 per word and message vector (3.8 one at a time: each
 // read serves half the work, measured 1.5x) and 10 for the seed word, the dot
 // product, the ring and the maximum; resident warps share the issue slots,
-// and fewer than three blocks do not fill them.  Registers decide the resident
+// and three blocks or fewer do not fill them (28 x 96, four lanes: three 637
+// us, five 580).  Registers decide the resident
 // blocks (half_min_blocks), or the shared memory of the S regions.  Measured
 // against the other group sizes: 28 x 256, d = 1, four lanes 1.30 ms, eight
 // 1.47; 24 x 128 two lanes 0.090, four 0.096, eight 0.100.
@@ -296,7 +297,7 @@ static bool half_split_choose(const int64_t* a, int R, int C, int d, int margina
       // of a seed (rows x words) in walks of about rounds / 4 high indices
       const double work = (double)Bp * ((K == 2 ? 2.5 : 3.8) * d * W + 10.0) + 6.0 * d * W + 60.0 +
                           1.5 * d * (F - k) * W / std::max(1.0, rounds * K / 4.0);
-      const double t = rounds * K * work * std::max(bps, 3.0);
+      const double t = rounds * K * work * std::max(bps, 3.4);
       cands.push_back({t, S, W, k});
     }
   }
