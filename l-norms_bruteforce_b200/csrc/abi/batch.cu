@@ -595,7 +595,19 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
   cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->dmem + b->off_heads, 0, sizeof(unsigned int) * std::max<size_t>(1, b->classes.size()), s);
   if (e == cudaSuccess) e = cudaEventRecord(b->fork, s);
-  for (auto& c : b->classes) {
+  // the classes whose CTAs have the most words to do first: the others fill
+  // the SMs beside them and as they end (256 matrices of 16-24 rows, three
+  // sets: 3.78 -> 3.65, 3.27 -> 3.03, 3.21 -> 2.83 ms)
+  std::vector<std::pair<double, size_t>> order;
+  for (size_t i = 0; i < b->classes.size(); ++i) {
+    const BatchClass& c = b->classes[i];
+    double words = 0;
+    for (int p : c.probs) words += (double)b->evaluated[p] * c.D * (c.HW > 0 ? c.HW : c.WB + c.WA);
+    order.push_back({-words / class_grid(c), i});
+  }
+  std::sort(order.begin(), order.end());
+  for (const auto& [unused, ci] : order) {
+    BatchClass& c = b->classes[ci];
     if (e != cudaSuccess) break;
     e = cudaStreamWaitEvent(c.stream, b->fork, 0);
     ld::BatchArgs args = class_args(c);
