@@ -192,9 +192,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
   extern __shared__ __align__(1024) unsigned char tc_mem[];
   block_start();
   // Per set: two chunks, one accumulator buffer, and four slots for the bases
-  // of its tiles (their four partial sums per row) and its walks.  A slot is
-  // written when the tile's first chunk is taken: then the products of the
-  // tile before last are done, so the epilogue is past the one before that.
+  // of its tiles (their four partial sums per row) and its walks.  A base slot
+  // is written when the tile's first chunk is taken: then the products of the
+  // tile before last are done, so the epilogue is past the one before that.  A
+  // group's walks are written one tile earlier, with the chunks of the tile
+  // before taken: the epilogue is then past tile T - 4, whose group (of one
+  // tile) had the slot.  It reads all three before it releases the tile.
   __shared__ __align__(8) uint64_t chunk_full[kSets][2], chunk_empty[kSets][2];
   __shared__ __align__(8) uint64_t slot_full[kSets][4], acc_full[kSets], acc_empty[kSets], drained;
   __shared__ unsigned long long s_high[kSets][4][128], s_next[kSets];   // first high index of a group's walks
@@ -530,6 +533,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
       if (!tc::bar_wait(&slot_full[g][slot], (tile / 4) & 1u, &s_abort)) break;
       const uint2 part = s_base[g][slot][row];
       const unsigned where = s_where[g][slot];
+      const unsigned long long high = s_high[g][where >> 30][row];
       const bool end = (unsigned)*(volatile int*)&s_end[g] == tile + 1u;
       if (!(kChunks <= 2 ? tc::bar_wait(&chunk_empty[g][last & 1u], (last / 2) & 1u, &s_abort)
                          : tc::bar_wait(&acc_full[g], tile & 1u, &s_abort)) || end)
@@ -556,7 +560,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
                     (max(max(m0, m1), max(m2, m3)) >> 6);
       if (v >= best) {
         // rows past the last walk repeat it, at its indices
-        const unsigned long long h = s_high[g][where >> 30][row] + (where & 0x3fffffffu);
+        const unsigned long long h = high + (where & 0x3fffffffu);
         if (v > best || h < best_high) { best = v; best_high = h; }
       }
     }
