@@ -39,6 +39,7 @@ bool tc_layout(const int64_t* a, int R, int C, int d, int marginal, int k, TcLay
   const int L = std::max(1, d - 1);
   const int P = V * C;
   if (d < 1 || d > 4 || P > 16 * ld::kTcMaxWords) return false;
+  if (d >= 3 && R - 1 - k > 32) return false;   // the kernel holds a walk's labels in 64 bits, two for each high row
   std::vector<Pair> pairs;
   std::vector<Feature> feats;
   pairs.reserve(P);

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
   __shared__ __align__(8) uint64_t chunk_full[kSets][2], chunk_empty[kSets][2];
   __shared__ __align__(8) uint64_t slot_full[kSets][4], acc_full[kSets], acc_empty[kSets], drained;
   __shared__ unsigned long long s_high[kSets][4][128], s_next[kSets];   // first high index of a group's walks
-  __shared__ unsigned long long s_label[kSets][128];                     // labels of their high rows, two bits each
+  __shared__ unsigned long long s_label[kSets][128];                     // labels of their high rows, two bits each (32 rows; d <= 2: one)
   __shared__ __align__(8) uint2 s_base[kSets][4][128];                    // four 16-bit partial sums
   __shared__ unsigned s_where[kSets][4];                                 // group and offset of a tile
   __shared__ int s_end[kSets], s_go[kSets];

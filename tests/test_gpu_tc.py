@@ -97,3 +97,17 @@ def test_a_block_of_ties(ld):
     ref = O.enumerate_max(a, 1, False)
     sol, desc = _solve(ld, a, 1, False)
     assert (sol.value, sol.gray_index) == ref, desc
+
+
+@pytest.mark.parametrize("rows", [38, 39, 40])
+def test_at_most_32_high_rows_with_three_labels(ld, rows):
+    """The kernel keeps a walk's labels in 64 bits, two per high row: more than
+    32 high rows stay with the table kernel.  (With 33 and 34 high rows, shards
+    beyond the first third of the range reported values that their labels do
+    not have: 152 for 88.)  The plans are only described: such a shard is long."""
+    a = _matrix(np.random.default_rng(rows), 3, 12, "pm1", rows)
+    for index in (0, 2 ** 30, 2 ** 31 - 2):
+        plan = ld.Plan(a, 3, False, ld.options(shard_index=index, shard_count=2 ** 31 - 1))
+        desc = plan.describe()
+        plan.close()
+        assert (_tc(desc) > 0) == (rows - 1 - 5 <= 32), desc
