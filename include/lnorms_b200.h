@@ -117,6 +117,10 @@ typedef struct {
                                    (measured: no faster replay on the 4096-
                                    matrix batch, 4x the creation time); 0 = the
                                    largest table that fits                   */
+    int32_t wait_polls;         /* tensor-core form: polls (of about 3 us) of a
+                                   device-side wait before the solve fails with
+                                   LD_ERR_TIMEOUT; 0 = 2^20; -1 = none, every
+                                   wait gives up at once (to test callers)   */
     void *stream;               /* cudaStream_t, NULL = the plan's own stream      */
 } ld_options;
 

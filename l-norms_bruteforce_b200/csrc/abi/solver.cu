@@ -595,6 +595,7 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
   if (R > ld_max_rows_for(d)) return ld_fail(LD_ERR_LIMIT, "%d rows exceed %d for d=%d", R, ld_max_rows_for(d), d);
   if (o.shard_count < 0 || (o.shard_count > 1 && (o.shard_index < 0 || o.shard_index >= o.shard_count)))
     return ld_fail(LD_ERR_ARG, "shard %d of %d", o.shard_index, o.shard_count);
+  if (o.wait_polls < -1) return ld_fail(LD_ERR_ARG, "wait_polls must be -1, 0 or positive (got %d)", o.wait_polls);
   const unsigned long long total = ld_labelings(R, d);
   if (total >= (1ull << 63)) return ld_fail(LD_ERR_LIMIT, "%d rows give 2^63 or more labelings", R);
   DeviceInfo di;
@@ -605,6 +606,7 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
   ld_plan* p = new ld_plan();
   p->device = o.device;
   p->R = R; p->C = C; p->d = d; p->marginal = marginal;
+  p->wait_polls = o.wait_polls == 0 ? ld::kTcWaitPolls : (unsigned)std::max(0, o.wait_polls);
   p->total = total;
   p->bounds = compute_bounds(a, R, C, marginal);
   st = choose_kernel(a, R, C, d, marginal, p->bounds, o, di.sms, &p->ch);
@@ -944,6 +946,7 @@ ld_status ldsolve::plan_enqueue(ld_plan* p) {
       targs.sym_words = p->sym_digits > 0 ? (int)ld_sym_table_len(p->d, p->sym_digits) : 0;
       targs.sym_table = args.sym_table;
       targs.value_offset = p->value_offset;
+      targs.wait_polls = p->wait_polls;
       targs.red = p->red;
       void* params[] = {&targs};
       LD_CUDA(cudaLaunchKernel(p->kfn, dim3(p->blocks), dim3(p->tpb), params, p->smem, r->stream));

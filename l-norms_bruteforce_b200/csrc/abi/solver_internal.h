@@ -132,7 +132,8 @@ struct ld_plan {
   size_t off_tot = 0, off_h0 = 0, off_tb = 0, off_A = 0;
   int Bp = 0, span = 0;                           // column split: table entries, words per slice region
   int pack16 = 0;                                 // table kernel: packed 16-bit maxima
-  size_t off_tc[10] = {};                          // tensor-core form: image offsets (TcArgs' order)
+  size_t off_tc[10] = {};                          // tensor-core form: image offsets (TcArgs' order),
+  unsigned wait_polls = 0;                        // polls of a wait
   bool uploaded = false;       // the upload belongs to the next fetched launch
   ld::Reduce red{};
   const void* kfn = nullptr;

@@ -41,8 +41,9 @@
 //       smallest high index attaining the thread's maximum.
 // The block position of the maximum is found once, by the last CTA.
 //
-// Every wait is bounded; one that runs out makes all warps leave, TMEM is
-// given back, and the result is LLONG_MAX (the host's LD_ERR_TIMEOUT).
+// Every wait is bounded (wait_polls); one that runs out makes all warps leave,
+// TMEM is given back when the products in flight are done, and the result is
+// LLONG_MAX (the host's LD_ERR_TIMEOUT).
 #pragma once
 #include "table_kernel.cuh"
 
@@ -80,8 +81,10 @@ struct TcArgs {
   int sym_words;                              // 64-bit completion counts
   const unsigned long long* sym_table;
   long long value_offset;
+  unsigned wait_polls;                        // of every wait but the last, for the products in flight
   Reduce red;
 };
+constexpr unsigned kTcWaitPolls = 1u << 20;   // of up to about 3 us
 
 __host__ __device__ inline size_t tc_align(size_t x) { return (x + 127) & ~(size_t)127; }
 
@@ -99,8 +102,6 @@ __host__ __device__ inline TcSmem tc_smem(int N, int steps, int rows, int labels
 }
 
 namespace tc {
-
-constexpr unsigned kWaitLimit = 1u << 20;   // polls of up to about 3 us
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -129,9 +130,9 @@ __device__ __forceinline__ void commit(uint64_t* b) {
 // lanes of a warp call it together.  (With one lane polling, or a time limit
 // on the blocking poll, the enumeration measured 6 to 40 % slower; polling two
 // barriers at once by half of the lanes each, 40 %.)
-__device__ __forceinline__ bool bar_wait(uint64_t* b, unsigned phase, int* abort) {
+__device__ __forceinline__ bool bar_wait(uint64_t* b, unsigned phase, int* abort, unsigned polls) {
   const uint32_t a = smem_addr(b);
-  for (unsigned n = 0; n < kWaitLimit; ++n) {
+  for (unsigned n = 0; n < polls; ++n) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
     unsigned tile = 0, chunk = 0, group = 0;         // of this set
     bool ok = true;
     auto take = [&] {
-      if (chunk >= 2) ok = tc::bar_wait(&chunk_empty[set][chunk & 1u], (chunk / 2 - 1) & 1u, &s_abort) && ok;
+      if (chunk >= 2) ok = tc::bar_wait(&chunk_empty[set][chunk & 1u], (chunk / 2 - 1) & 1u, &s_abort, a.wait_polls) && ok;
     };
     auto hand = [&] {
       __syncwarp();
@@ -483,10 +484,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
 #pragma unroll
       for (int n = 0; n < kChunks; ++n, ++chunk) {
         const unsigned c = chunk & 1u;
-        ok = tc::bar_wait(&chunk_full[g][c], (chunk / 2) & 1u, &s_abort);
+        ok = tc::bar_wait(&chunk_full[g][c], (chunk / 2) & 1u, &s_abort, a.wait_polls);
         if (!ok) break;
         if (n == 0) {
-          if (tile >= 1) ok = tc::bar_wait(&acc_empty[g], (tile - 1) & 1u, &s_abort);
+          if (tile >= 1) ok = tc::bar_wait(&acc_empty[g], (tile - 1) & 1u, &s_abort, a.wait_polls);
           if (!ok) break;
           if ((unsigned)*(volatile int*)&s_end[g] == tile + 1u) {
             // the set's last, empty tile: the epilogue waits for it as for others
@@ -519,7 +520,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
     if (tc::elect()) tc::commit(&drained);
     __syncwarp();
     int never = 0;
-    tc::bar_wait(&drained, 0u, &never);
+    tc::bar_wait(&drained, 0u, &never, kTcWaitPolls);
   } else {
     // ---- epilogue: row tid % 128 of a set's tiles
     const int row = tid & 127, g = warp >> 2;
@@ -530,13 +531,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
       // complete (with three chunks a tile that release could be two phases of
       // its barrier away, which one parity bit does not tell apart)
       const unsigned slot = tile & 3u, last = tile * kChunks + kChunks - 1;
-      if (!tc::bar_wait(&slot_full[g][slot], (tile / 4) & 1u, &s_abort)) break;
+      if (!tc::bar_wait(&slot_full[g][slot], (tile / 4) & 1u, &s_abort, a.wait_polls)) break;
       const uint2 part = s_base[g][slot][row];
       const unsigned where = s_where[g][slot];
       const unsigned long long high = s_high[g][where >> 30][row];
       const bool end = (unsigned)*(volatile int*)&s_end[g] == tile + 1u;
-      if (!(kChunks <= 2 ? tc::bar_wait(&chunk_empty[g][last & 1u], (last / 2) & 1u, &s_abort)
-                         : tc::bar_wait(&acc_full[g], tile & 1u, &s_abort)) || end)
+      if (!(kChunks <= 2 ? tc::bar_wait(&chunk_empty[g][last & 1u], (last / 2) & 1u, &s_abort, a.wait_polls)
+                         : tc::bar_wait(&acc_full[g], tile & 1u, &s_abort, a.wait_polls)) || end)
         break;
       tc::fence_after();
       int m0 = INT_MIN, m1 = INT_MIN, m2 = INT_MIN, m3 = INT_MIN;

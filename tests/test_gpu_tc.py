@@ -26,6 +26,12 @@ def _tc(desc):
     return int(desc.split("tc=")[1].split()[0])
 
 
+def _chunks(desc):
+    """Chunks per tile (tc_chunk_steps); 0 without the tensor-core form."""
+    steps = _tc(desc) // 16
+    return 0 if steps == 0 else 1 if steps <= 16 else -(-steps // (12 if steps in (22, 24) else 10))
+
+
 def _matrix(rng, d, cols, kind, rows=0):
     shape = (rows or ROWS[d], cols)
     if kind == "pm1":
@@ -111,3 +117,32 @@ def test_at_most_32_high_rows_with_three_labels(ld, rows):
         desc = plan.describe()
         plan.close()
         assert (_tc(desc) > 0) == (rows - 1 - 5 <= 32), desc
+
+
+@pytest.mark.parametrize("d,marg,cols,chunks", [(1, False, 16, 1), (1, False, 33, 2), (1, True, 48, 3), (2, False, 16, 1),
+                                                (2, False, 24, 2), (3, False, 17, 1), (3, False, 30, 3), (4, False, 21, 2)])
+def test_a_wait_that_runs_out(ld, d, marg, cols, chunks):
+    """Waits that give up at once: the plan and the one-shot solve fail with
+    LD_ERR_TIMEOUT, and the next solves are right.  Waits of one poll may run
+    out anywhere: the solve fails in the same way or is right."""
+    a = _matrix(np.random.default_rng(cols), d, cols, "pm1")
+    ref = O.enumerate_max(a, d, marg)
+    good = ld.Plan(a, d, marg)
+    assert _chunks(good.describe()) == chunks, good.describe()
+    for polls in (-1, 1):
+        plan = ld.Plan(a, d, marg, ld.options(wait_polls=polls))
+        for solve in (plan.solve, plan.solve, lambda: ld.solve_reduced(a, d, marg, ld.options(wait_polls=polls))):
+            try:
+                sol = solve()
+                assert polls == 1 and (sol.value, sol.gray_index) == ref
+            except ld.LdError as e:
+                assert e.status == 7
+            sol = good.solve()
+            assert (sol.value, sol.gray_index) == ref
+        plan.close()
+    good.close()
+    sol = ld.solve_reduced(a, d, marg)
+    assert (sol.value, sol.gray_index) == ref
+    with pytest.raises(ld.LdError) as e:
+        ld.Plan(a, d, marg, ld.options(wait_polls=-2))
+    assert e.value.status == 1
