@@ -678,6 +678,9 @@ extern "C" ld_status ld_batch_results(ld_batch* b, int64_t* values, uint64_t* gr
   if (!b->launched) return ld_fail(LD_ERR_ARG, "batch has not been launched");
   LD_CUDA(cudaSetDevice(b->device));
   LD_CUDA(cudaStreamSynchronize(b->stream));
+  for (int p = 0; p < b->n; ++p)
+    if (b->plans[p] && wait_ran_out(b->plans[p], b->hres[p]))
+      return ld_fail(LD_ERR_TIMEOUT, "batch entry %d: a device-side wait of the tensor-core enumeration ran out", p);
   for (int p = 0; p < b->n; ++p) {
     values[p] = b->hres[p].value;
     if (gray_indices) gray_indices[p] = b->hres[p].index;

@@ -1024,7 +1024,7 @@ ld_status ldsolve::plan_fetch(ld_plan* p, ld_result* res, int32_t* strategy) {
     LD_CUDA(cudaEventElapsedTime(&ms, r->ev0, r->ev1));
     h = *copy;
   }
-  if (p->ch.kind == LD_KERNEL_TABLE && p->ch.tc && h.value == LLONG_MAX)
+  if (wait_ran_out(p, h))
     return ld_fail(LD_ERR_TIMEOUT, "tensor-core enumeration: a device-side wait ran out");
   memset(res, 0, sizeof *res);
   res->value = h.value;

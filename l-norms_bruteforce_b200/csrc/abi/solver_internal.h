@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstddef>
 #include <cstdint>
 #include <mutex>
@@ -153,6 +154,11 @@ ld_status plan_build(const int64_t* a, int R, int C, int d, int marginal, const 
                      Resources* shared, ld_plan** out, bool one_shot = false);
 ld_status plan_enqueue(ld_plan* p);
 unsigned long long plan_evaluated(const ld_plan* p);
+// Whether a result slot of the plan's says that a wait of its kernel ran out
+// (tc_kernel.cuh; no value is LLONG_MAX).  To be asked wherever one is read.
+inline bool wait_ran_out(const ld_plan* p, const ld::Slot& s) {
+  return p->ch.kind == LD_KERNEL_TABLE && p->ch.tc && s.value == LLONG_MAX;
+}
 ld_status plan_fetch(ld_plan* p, ld_result* res, int32_t* strategy);
 
 }  // namespace ldsolve

@@ -4,6 +4,8 @@ Gray index) for d = 1, LM, 2, 3 and 4, over column counts at the edges of the
 byte words, +-1 entries (ties, both parities of a column's sum), entries to
 +-3, one-sided columns, equal rows, zero columns, shards, label symmetry on
 and off, repeated launches of a plan, and inside a batch."""
+import contextlib
+
 import numpy as np
 import pytest
 
@@ -146,3 +148,33 @@ def test_a_wait_that_runs_out(ld, d, marg, cols, chunks):
     with pytest.raises(ld.LdError) as e:
         ld.Plan(a, d, marg, ld.options(wait_polls=-2))
     assert e.value.status == 1
+
+
+@contextlib.contextmanager
+def ld_batch(ld, mats, ds, tune, **kw):
+    b = ld.Batch(mats, ds, opts=ld.options(**kw), autotune=tune)
+    try:
+        yield b
+    finally:
+        b.close()
+
+
+@pytest.mark.parametrize("tune", [False, True])
+def test_inside_a_batch(ld, tune):
+    """Batch entries that get their own plan take the tensor-core form too; a
+    wait that runs out there fails the batch instead of being its value."""
+    rng = np.random.default_rng(44)
+    mats = [_matrix(rng, 4, 21, "pm1"), rng.integers(-90, 91, size=(12, 20)).astype(np.int64), _matrix(rng, 4, 8, "amp3"),
+            _matrix(rng, 4, 20, "pm1", 11)]
+    ds = [4, 1, 4, 4]
+    refs = [O.enumerate_max(a, d, False) for a, d in zip(mats, ds)]
+    assert _tc(_solve(ld, mats[0], 4, False)[1]) > 0
+    with ld_batch(ld, mats, ds, tune) as b:
+        for _ in range(2):
+            v, g, _ = b.solve()
+            assert [(int(x), int(y)) for x, y in zip(v, g)] == refs, b.describe()
+    with ld_batch(ld, mats, ds, tune, wait_polls=-1) as b:
+        for _ in range(2):
+            with pytest.raises(ld.LdError) as e:
+                b.solve()
+            assert e.value.status == 7 and "entry 0" in str(e.value)
