@@ -273,7 +273,9 @@ ld_status ld_plan_describe(const ld_plan *plan, char *buf, size_t cap);
 void *ld_plan_stream(const ld_plan *plan);
 /* Device address of the plan's 16-byte result {int64 value; uint64 index},
  * valid after a launch completes on the plan's stream (for callers that
- * combine shards on the device, e.g. with an NCCL all-reduce). */
+ * combine shards on the device, e.g. with an NCCL all-reduce).  The value
+ * INT64_MAX is no result: a device-side wait ran out, for which
+ * ld_plan_result returns LD_ERR_TIMEOUT. */
 void *ld_plan_result_device(const ld_plan *plan);
 void ld_plan_destroy(ld_plan *plan);
 

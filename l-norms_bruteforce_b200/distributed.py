@@ -32,7 +32,9 @@ def combine_tensor(val_idx, group=None):
     tensor (value, Gray index) per rank, without leaving the device: two
     all-reduces (MAX on the value, MIN on the index of the ranks at the
     maximum) queued on the current stream.  Returns two 1-element tensors.
-    Gray indices are below 2^63, so an index read as int64 keeps its order."""
+    Gray indices are below 2^63, so an index read as int64 keeps its order.
+    A rank whose kernel gave up a wait holds INT64_MAX, which wins on every
+    rank: read the tensors with `combined`."""
     import torch
     import torch.distributed as dist
 
@@ -43,14 +45,24 @@ def combine_tensor(val_idx, group=None):
     return v, i
 
 
+def combined(v, i) -> tuple[int, int]:
+    """The (value, index) that combine_tensor returned, as integers.  Raises
+    LdError (LD_ERR_TIMEOUT) on every rank when a wait ran out on one."""
+    from . import LdError
+
+    value, index = int(v.item()), int(i.item())
+    if value == INT64_MAX:
+        raise LdError(7, "a device-side wait ran out on a rank: the combined solve has no result")
+    return value, index
+
+
 def combine(value: int, index: int, group=None, device=None) -> tuple[int, int]:
     """Global (max value, smallest index attaining it) over the ranks, from
     host integers (combine_tensor on a tensor of the given device)."""
     import torch
 
     dev = device if device is not None else "cpu"
-    v, i = combine_tensor(torch.tensor([value, index], dtype=torch.int64, device=dev), group=group)
-    return int(v.item()), int(i.item())
+    return combined(*combine_tensor(torch.tensor([value, index], dtype=torch.int64, device=dev), group=group))
 
 
 def solve_sharded(ld, a, d: int, marginal: bool, rank: int, world: int, device: int = 0,

@@ -109,6 +109,43 @@ def test_failed_rank_surfaces_as_an_error():
     assert res[0][0] == "error"                # the survivor's exchange errors out, it does not hang
 
 
+def _rank_without_result(rank, world, port, out):
+    import datetime
+
+    sys.path.insert(0, str(ROOT / "tests"))
+    import torch
+    import torch.distributed as dist
+    from conftest import load_package
+
+    load_package()
+    import lnorms_b200.distributed as D
+
+    dist.init_process_group("gloo", init_method=f"tcp://127.0.0.1:{port}", rank=rank, world_size=world,
+                            timeout=datetime.timedelta(seconds=10))
+    # rank 1's kernel gave up a wait: its device result is (INT64_MAX, 0)
+    mine = (100 + rank, 7) if rank != 1 else (np.iinfo(np.int64).max, 0)
+    got = []
+    for read in (lambda: D.combine(*mine), lambda: D.combined(*D.combine_tensor(torch.tensor(mine, dtype=torch.int64)))):
+        try:
+            got.append(("value", read()))
+        except Exception as e:
+            got.append((type(e).__name__, getattr(e, "status", None)))
+    out.put((rank, got))
+    dist.destroy_process_group()
+
+
+def test_a_rank_without_a_result_fails_every_rank():
+    ctx = mp.get_context("spawn")
+    out, port = ctx.Queue(), _free_port()
+    procs = [ctx.Process(target=_rank_without_result, args=(r, 3, port, out)) for r in range(3)]
+    for p in procs:
+        p.start()
+    res = dict(out.get(timeout=120) for _ in procs)
+    for p in procs:
+        p.join(timeout=60)
+    assert all(res[r] == [("LdError", 7)] * 2 for r in range(3)), res
+
+
 def test_shard_bounds_tile():
     sys.path.insert(0, str(ROOT))
     from conftest import load_package
