@@ -892,8 +892,7 @@ ld_status ldsolve::plan_build(const int64_t* a, int R, int C, int d, int margina
                     ? (unsigned long long*)(base_ptr + kOffWork) : nullptr;
   if (one_shot) {
     p->host = (ld::HostSlot*)((char*)p->res->hstage + off_host);
-    p->red.host = p->host;
-    p->red.start = (unsigned long long*)(base_ptr + kOffStart);
+    memcpy(image.data() + kOffHost, &p->host, sizeof p->host);
   }
   memcpy(p->res->hstage, image.data(), p->upload_bytes);
   cudaError_t ce = cudaMemcpyAsync(p->res->dmem, p->res->hstage, p->upload_bytes, cudaMemcpyHostToDevice,

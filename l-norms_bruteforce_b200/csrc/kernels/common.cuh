@@ -33,9 +33,23 @@ struct Reduce {
   Slot* result;
   unsigned long long* work;   // walk counter the launch's warps fetch from (0 before
                               // the launch, reset by the last block), or null
-  HostSlot* host = nullptr;   // also write the result here
-  unsigned long long* start = nullptr;   // with host: ULLONG_MAX before the launch, re-armed likewise
 };
+
+// A one-shot solve's two further words of the scratch header, at these 64-bit
+// words from `counter`: the first block's start time (ULLONG_MAX before the
+// launch, re-armed likewise), and where the last block also writes the result
+// and the times (null: nowhere; so the header's words must be zero elsewhere).
+// Not members: with two pointers more the wide kernel's arguments were above
+// 128 bytes, which the compiler handles differently, and its loops got other
+// registers (24 x 300, d = 1: 48 instead of 63 and 2.12 ms instead of 1.86; 17
+// x 2048, d = 2: 683 us instead of 593 even at 128 bytes).
+constexpr int kStartWord = 5, kHostWord = 6;
+__device__ __forceinline__ unsigned long long* start_word(const Reduce& R) {
+  return reinterpret_cast<unsigned long long*>(R.counter) + kStartWord;
+}
+__device__ __forceinline__ HostSlot* host_slot(const Reduce& R) {
+  return reinterpret_cast<HostSlot*>(reinterpret_cast<unsigned long long*>(R.counter)[kHostWord]);
+}
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -142,6 +156,7 @@ __device__ __forceinline__ bool grid_reduce(long long v, unsigned long long n, c
   __shared__ bool s_last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int nwarps = (blockDim.x + 31) >> 5;
+  HostSlot* host = threadIdx.x == 0 ? host_slot(R) : nullptr;
   warp_best(v, n);
   if (lane == 0) { s_v[wid] = v; s_n[wid] = n; }
   __syncthreads();
@@ -153,7 +168,7 @@ __device__ __forceinline__ bool grid_reduce(long long v, unsigned long long n, c
       R.slots[blockIdx.x].value = v;
       R.slots[blockIdx.x].index = n;
       if (v != LLONG_MIN) atomicMax(R.gvalue, v);
-      if (R.host) atomicMin(R.start, block_clock());
+      if (host) atomicMin(start_word(R), block_clock());
       __threadfence();
       unsigned int done = atomicAdd(R.counter, 1u);
       s_last = (done == gridDim.x - 1);
@@ -179,9 +194,7 @@ __device__ __forceinline__ bool grid_reduce(long long v, unsigned long long n, c
     for (int w = 0; w < nwarps; ++w) if (s_n[w] < best) best = s_n[w];
     R.result->value = gmax;
     R.result->index = best;
-    if (R.host) {
-      *R.host = HostSlot{gmax, best, atomicExch(R.start, ULLONG_MAX), global_ns()};
-    }
+    if (host) *host = HostSlot{gmax, best, atomicExch(start_word(R), ULLONG_MAX), global_ns()};
     *R.gvalue = LLONG_MIN;
     *R.counter = 0u;
     if (R.work) *R.work = 0ull;   // every block has finished fetching walks

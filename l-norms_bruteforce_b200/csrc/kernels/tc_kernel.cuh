@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const TcArgs a) {
   if (tid == 0) {
     const unsigned long long n = gh * (unsigned long long)a.B + (unsigned long long)s_first;
     a.red.result->index = n;
-    if (a.red.host) { a.red.host->index = n; a.red.host->t1 = global_ns(); }
+    if (HostSlot* host = host_slot(a.red)) { host->index = n; host->t1 = global_ns(); }
   }
 }
 

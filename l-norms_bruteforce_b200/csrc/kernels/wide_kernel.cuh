@@ -33,6 +33,7 @@ struct WideArgs {
   unsigned long long rank_begin, rank_end;
   Reduce red;
 };
+static_assert(sizeof(WideArgs<int>) <= 120, "larger arguments change the loops' registers (common.cuh)");
 
 constexpr int kWideThreads = 128;
 
