@@ -36,16 +36,19 @@ size_t gemm_smem() {
   return tiles > cap ? tiles : cap;
 }
 
-// Shared-memory limits of the three GEMM instances; called before any
+// Shared-memory limits of the GEMM instances; called before any
 // launch on the current device (and before any stream capture).
 cudaError_t gemm_init() {
-  cudaError_t e = cudaFuncSetAttribute(ld::mlp::tc_gemm_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(ld::mlp::tc_gemm_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)gemm_smem<64>());
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(ld::mlp::tc_gemm_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(ld::mlp::tc_gemm_kernel<64, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)gemm_smem<64>());
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(ld::mlp::tc_gemm_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)gemm_smem<128>());
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(ld::mlp::tc_gemm_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(ld::mlp::tc_gemm_kernel<256, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)gemm_smem<256>());
   return e;
 }
@@ -53,9 +56,7 @@ cudaError_t gemm_init() {
 template <int BN>
 cudaError_t launch_gemm(const ld::mlp::GemmArgs& g, cudaStream_t s) {
   dim3 grid(g.M / ld::mlp::kTileM, g.N / BN);
-  ld::mlp::GemmGroup group{};
-  group.g[0] = g;
-  ld::mlp::tc_gemm_kernel<BN><<<grid, 128, gemm_smem<BN>(), s>>>(group);
+  ld::mlp::tc_gemm_kernel<BN, 1><<<grid, 128, gemm_smem<BN>(), s>>>(ld::mlp::GemmGroup<1>{{g}});
   return cudaGetLastError();
 }
 
@@ -185,12 +186,12 @@ cudaError_t enqueue_backward(ld_mlp* n) {
   if ((e = gemm(n->dZ2, n->W2T, B, kHid, kHid, nullptr, nullptr, n->dZ1T, nullptr, 0, n->err, n->s, n->H1)) != cudaSuccess) return e;
   // the weight gradients in one launch; W3: [kOutGP x B] x [kHid x B]^T (rows
   // kOutP.. of dZ3T are zero)
-  ld::mlp::GemmGroup w{};
+  ld::mlp::GemmGroup<3> w{};
   w.g[0] = ld::mlp::GemmArgs{n->dZ3T, n->H2T, kOutGP, kHid, B, n->gW3, nullptr, nullptr, nullptr, 0, n->err, nullptr};
   w.g[1] = ld::mlp::GemmArgs{n->dZ2T, n->H1T, kHid, kHid, B, n->gW2, nullptr, nullptr, nullptr, 0, n->err, nullptr};
   w.g[2] = ld::mlp::GemmArgs{n->dZ1T, n->XT, kHid, kInP, B, n->gW1, nullptr, nullptr, nullptr, 0, n->err, nullptr};
   const dim3 grid(kHid / ld::mlp::kTileM, kHid / 64, 3);
-  ld::mlp::tc_gemm_kernel<64><<<grid, 128, gemm_smem<64>(), n->s>>>(w);
+  ld::mlp::tc_gemm_kernel<64, 3><<<grid, 128, gemm_smem<64>(), n->s>>>(w);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const ld::mlp::BiasGrads bias{{n->dZ1T, n->dZ2T, n->dZ3T}, {n->gb1, n->gb2, n->gb3}, {kHid, kHid, kOutP}};
   ld::mlp::bias_grad_kernel<<<(2 * kHid + kOutP) / 4, 128, 0, n->s>>>(bias, B);

@@ -80,8 +80,12 @@ struct GemmArgs {
 
 // Up to three products in one launch (blockIdx.z): the weight gradients, which
 // are 4, 8 and 2 tiles of 128 x 64 with all of the batch to add up (three
-// launches of 22 us each, one of 20).
-struct GemmGroup { GemmArgs g[3]; };
+// launches of 22 us each, one of 20).  A single product has an instance of its
+// own: through the arguments of three (264 bytes, indexed at run time; 40
+// registers instead of 80) a forward pass of 1024 rows took 97 us, not 90.
+template <int P>
+struct GemmGroup { GemmArgs g[P]; };
+static_assert(sizeof(GemmGroup<1>) <= 128, "larger arguments cost the single product its registers");
 
 // Stages: these products are short chains of chunks on few SMs (of 20 us for
 // K = 1024, 9 are there for a single chunk too).  Four 64-wide stages instead
@@ -100,10 +104,10 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // stage, the CTA's threads copy the next chunks into the others with cp.async.
 // A stage is refilled only after the mbarrier of the MMAs that read it has
 // completed.
-template <int BN>
-__global__ void __launch_bounds__(128) tc_gemm_kernel(const GemmGroup group) {
-  const GemmArgs& g = group.g[blockIdx.z];
-  if ((int)blockIdx.x * kTileM >= g.M || (int)blockIdx.y * BN >= g.N) return;   // outside this product
+template <int BN, int P>
+__global__ void __launch_bounds__(128) tc_gemm_kernel(const GemmGroup<P> group) {
+  const GemmArgs& g = group.g[P > 1 ? blockIdx.z : 0];
+  if (P > 1 && ((int)blockIdx.x * kTileM >= g.M || (int)blockIdx.y * BN >= g.N)) return;   // outside this product
   constexpr int kStages = gemm_stages(BN);
   static_assert(BN == 64 || BN == 128 || BN == 256, "tile width");
   constexpr int kStageA = kTileM * kTileK * 2, kStageB = BN * kTileK * 2;
