@@ -356,7 +356,9 @@ int ld_cli_main(int argc, char **argv);
 /* atomically).  A later call with the same matrix, d, marginal, pieces and */
 /* enumerate_all continues after the last recorded piece; a checkpoint of   */
 /* another problem is refused (LD_ERR_ARG), and so is a piece that would    */
-/* not start where the recorded coverage ends (changed options or device).  */
+/* not start where the recorded coverage ends (changed options or device);  */
+/* one that does with pack16 = -1 runs so (a checkpoint begun before the    */
+/* 16-bit and tensor-core forms).                                           */
 /* At most max_pieces pieces run per call (<= 0: all).  *done = 1 once every */
 /* piece has run; res (and strategy, rows-1 labels) then hold what          */
 /* ld_solve_reduced gives, with labelings / evaluated / kernel_ms summed    */

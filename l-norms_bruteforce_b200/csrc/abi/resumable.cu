@@ -103,6 +103,15 @@ extern "C" ld_status ld_solve_resumable(const int64_t* a, int32_t rows, int32_t 
     if (st != LD_OK) return st;
     uint64_t lo = 0, hi = 0;
     ld_plan_range(p, &lo, &hi);
+    if (pieces > 1 && lo != ck.covered && o.pack16 == 0) {
+      // a checkpoint from before the 16-bit and tensor-core forms, whose walks
+      // may differ: it goes on with the kernels it was begun with
+      ld_plan_destroy(p);
+      po.pack16 = -1;
+      st = ld_plan_create(a, rows, cols, d, marg, &po, &p);
+      if (st != LD_OK) return st;
+      ld_plan_range(p, &lo, &hi);
+    }
     if (pieces > 1 && lo != ck.covered) {
       ld_plan_destroy(p);
       return ld_fail(LD_ERR_ARG, "piece %d starts at Gray index %llu, the checkpoint covers [0, %llu): the solve's "

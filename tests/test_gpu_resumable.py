@@ -52,3 +52,26 @@ def test_changed_geometry_is_refused(ld, tmp_path):
     # the checkpoint is untouched and the original options continue it
     done, sol = ld.solve_resumable(a, 3, False, pieces=5, checkpoint=ck, opts=ld.options(tile=1))
     assert done and (sol.value, sol.gray_index) == O.enumerate_max(a, 3, False)
+
+
+@pytest.mark.parametrize("d,shape,amp,pieces", [(1, (26, 33), 1, 7), (2, (26, 16), 1, 5), (3, (17, 17), 1, 5), (1, (22, 90), 40, 7),
+                                                (3, (10, 93), 300, 2), (3, (11, 100), 300, 3), (3, (12, 70), 300, 5),
+                                                (3, (13, 24), 300, 5), (3, (14, 18), 300, 5), (3, (14, 32), 20, 7)])
+def test_checkpoint_from_before_the_16_bit_and_tensor_core_forms(ld, tmp_path, d, shape, amp, pieces):
+    """pack16=-1 gives the kernels, and so the pieces, from before these forms.
+    Such a checkpoint is continued by a call with default options."""
+    rng = np.random.default_rng(shape[1])
+    a = rng.choice(np.array([-amp, amp]), size=shape) if amp == 1 else rng.integers(-amp, amp + 1, size=shape)
+    a = a.astype(np.int64)
+    plan = ld.Plan(a, d, False, ld.options(shard_index=1, shard_count=pieces, pack16=-1))
+    start = plan.range[0]
+    plan.close()
+    ck = tmp_path / "solve.ckpt"
+    done, _ = ld.solve_resumable(a, d, False, pieces=pieces, checkpoint=ck, max_pieces=1, opts=ld.options(pack16=-1))
+    assert not done and f"covered {start}" in ck.read_text()
+    if pieces > 2:
+        done, _ = ld.solve_resumable(a, d, False, pieces=pieces, checkpoint=ck, max_pieces=1)
+        assert not done and "next 2" in ck.read_text()
+    done, sol = ld.solve_resumable(a, d, False, pieces=pieces, checkpoint=ck)
+    assert done and (sol.value, sol.gray_index) == O.enumerate_max(a, d, False)
+    assert sol.labelings == O.total(shape[0], d)
