@@ -50,8 +50,8 @@ typedef struct {
                               L_CUDA.cu:80 strict '>' and :347 strict '<')          */
     uint64_t labelings;    /* labelings the solve covered (evaluated, or skipped by
                               a bound or by label symmetry)                        */
-    float kernel_ms;       /* device time of the solve's launches (plans and the
-                              pruned search: CUDA events; ld_solve_reduced: the
+    float kernel_ms;       /* device time of the solve's launches (plans: CUDA
+                              events; ld_solve_reduced and the pruned search: the
                               first block's start to the last one's end)           */
     int32_t kernel_kind;   /* LD_KERNEL_* actually used                             */
     int32_t lane_bits;     /* 8, 32 or 64: arithmetic lane width used (32: also two
@@ -223,7 +223,7 @@ typedef struct {
     uint64_t highs_total, highs_visited, highs_kept;  /* high indices (blocks of `block` labelings) */
     uint64_t block;                           /* labelings per high index                */
     int64_t incumbent;                        /* value of the incumbent (INT64_MIN: none) */
-    float bound_ms, scan_ms;                  /* device time of the two launches          */
+    float bound_ms, scan_ms;                  /* device time: first bound, other launches */
     int32_t pruned;                           /* 1: pruned kernels ran; 0: plain fallback */
     int32_t low_rows, walk_rows;              /* rows tabulated / walked per prefix       */
 } ld_prune_stats;

@@ -184,7 +184,7 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
   const long long gmin = LLONG_MIN;
   memcpy(image.data() + 8, &gmin, sizeof gmin);
   const ld::Slot none{LLONG_MIN, ULLONG_MAX};
-  memcpy(image.data() + offBest, &none, sizeof none);   // then the high indices kept
+  memcpy(image.data() + offBest, &none, sizeof none);   // then the high indices kept, and the time
   pack_row(tot.data(), ch, (uint32_t*)(image.data() + offTot));
   pack_row(h0.data(), ch, (uint32_t*)(image.data() + offH0));
   pack_row(tb.data(), ch, (uint32_t*)(image.data() + offTb));
@@ -219,15 +219,16 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
   if (st != LD_OK) return st;
   char* dmem = (char*)r->dmem;
   cudaStream_t s = r->stream;
-  struct Best { ld::Slot slot; unsigned long long kept; };
+  struct Best { ld::Slot slot; unsigned long long kept, ns; };
+  struct Bounded { unsigned long long count, t0, t1; };   // PruneArgs::list_count
   Best* out_h = (Best*)r->hstage;
-  unsigned long long* hcount = (unsigned long long*)((char*)r->hstage + 64);
+  Bounded* out_b = (Bounded*)((char*)r->hstage + 64);
   float ms_b = 0.f, ms_s = 0.f;
   auto fail = [&](const char* what, cudaError_t e) {
     cudaStreamSynchronize(s);
     return ld_fail(LD_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   };
-  unsigned long long visited = 0, d2h = sizeof(Best);
+  unsigned long long visited = 0, h2d = upload, d2h = sizeof(Best);
   cudaError_t e;
   if ((e = cudaMemcpyAsync(dmem, image.data(), upload, cudaMemcpyHostToDevice, s)) != cudaSuccess) return fail("upload", e);
   {
@@ -265,32 +266,30 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
       args.run = run;
       t.walk_begin = begin; t.walk_end = end;
       const unsigned long long need = ((total + run - 1) / run + ld::kPruneThreads - 1) / ld::kPruneThreads;
-      cudaError_t x = cudaMemsetAsync(args.list_count, 0, 8, s);
+      cudaError_t x = cudaMemsetAsync(args.list_count, 0, sizeof(Bounded), s);
       if (x != cudaSuccess) return x;
       return cudaLaunchKernel(kb, dim3((unsigned)std::min(full_b, need)), dim3(ld::kPruneThreads), params, smem_b, s);
     };
-    if ((e = cudaEventRecord(r->ev0, s)) != cudaSuccess) return fail("event", e);
     unsigned long long* lists[2] = {(unsigned long long*)(dmem + off_a), (unsigned long long*)(dmem + off_b)};
     const unsigned long long caps[2] = {capA, capB};
     int cur = 0;                       // the list that holds the survivors
     args.src = nullptr; args.expand = walks; args.list = lists[0]; args.m_rest = m_walk;
     if ((e = bound(0, walks)) != cudaSuccess) return fail("walk bound launch", e);
-    if ((e = cudaEventRecord(r->ev1, s)) != cudaSuccess) return fail("event", e);
-    if ((e = cudaMemcpyAsync(hcount, args.list_count, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+    if ((e = cudaMemcpyAsync(out_b, args.list_count, sizeof(Bounded), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
       return fail("survivors", e);
     // the low rows' norm, meanwhile
     if ((st = rest_norm(a, C, d, marginal, k, o.device, &m_low)) != LD_OK) { cudaStreamSynchronize(s); return st; }
     m_low += kl;
     if ((e = cudaSetDevice(o.device)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
       return fail("walk bound", e);
-    unsigned long long n = *hcount;
+    unsigned long long n = out_b->count;
     ps.walks_kept = n;
-    d2h += 8;
+    ms_b = (float)(out_b->t1 - out_b->t0) * 1e-6f;
+    d2h += sizeof(Bounded);
     // When more than a quarter of the walks survive their bound the search
     // would do most of the plain enumeration's work at a lower rate: run the
     // plain enumeration instead (same result).
     if (o.prune_policy == 0 && n * 4ull > walks) {
-      cudaEventElapsedTime(&ms_b, r->ev0, r->ev1);
       ps.bound_ms = ms_b;
       return plain();
     }
@@ -317,6 +316,7 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
         if ((e = cudaMemcpyAsync(dmem + offTtop, tw.data(), WT * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
             (e = cudaStreamSynchronize(s)) != cudaSuccess)
           return fail("totals", e);
+        h2d += WT * 4;
       }
       args.src = lists[cur];
       args.list = lists[cur ^ 1];
@@ -326,12 +326,13 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
       const unsigned long long total = n * args.expand;
       if (left > 0) {
         if ((e = bound(0, total)) != cudaSuccess) return fail("level launch", e);
-        if ((e = cudaMemcpyAsync(hcount, args.list_count, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        if ((e = cudaMemcpyAsync(out_b, args.list_count, sizeof(Bounded), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
             (e = cudaStreamSynchronize(s)) != cudaSuccess)
           return fail("level bound", e);
-        n = *hcount;
+        n = out_b->count;
+        ms_s += (float)(out_b->t1 - out_b->t0) * 1e-6f;
         cur ^= 1;
-        d2h += 8;
+        d2h += sizeof(Bounded);
         continue;
       }
       // whole high indices: as many at once as the list can hold, a power of
@@ -345,13 +346,11 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
           return fail("evaluation launch", e);
       }
     }
-    if ((e = cudaEventRecord(r->ev2, s)) != cudaSuccess) return fail("event", e);
   }
   if ((e = cudaMemcpyAsync(out_h, dmem + offBest, sizeof(Best), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
     return fail("result", e);
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail("solve", e);
-  cudaEventElapsedTime(&ms_b, r->ev0, r->ev1);
-  cudaEventElapsedTime(&ms_s, r->ev1, r->ev2);
+  ms_s += (float)out_h->ns * 1e-6f;
   const ld::Slot out = out_h->slot;
   const unsigned long long kept = out_h->kept;
   if (ps.incumbent != LLONG_MIN && out.value < ps.incumbent)
@@ -364,7 +363,7 @@ extern "C" ld_status ld_solve_pruned(const int64_t* a, int32_t R, int32_t C, int
   res->kernel_ms = ms_b + ms_s;
   res->kernel_kind = LD_KERNEL_TABLE;
   res->lane_bits = ch.lane_bits;
-  res->h2d_bytes = upload;
+  res->h2d_bytes = h2d;
   res->d2h_bytes = d2h;
   res->evaluated = kept * (unsigned long long)B;   // high indices whose block was scanned
   if (strategy) ld_gray_labels(out.index, R, d, strategy);

@@ -509,7 +509,6 @@ void resources_release(Resources* r) {
   if (r->hstage) cudaFreeHost(r->hstage);
   if (r->ev0) cudaEventDestroy(r->ev0);
   if (r->ev1) cudaEventDestroy(r->ev1);
-  if (r->ev2) cudaEventDestroy(r->ev2);
   if (r->own_stream && r->stream) cudaStreamDestroy(r->stream);
   if (cur >= 0) cudaSetDevice(cur);
   *r = Resources();
@@ -524,7 +523,6 @@ ld_status resources_acquire(Resources* r, int device, cudaStream_t user_stream, 
     else { LD_CUDA(cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking)); r->own_stream = true; }
     LD_CUDA(cudaEventCreate(&r->ev0));
     LD_CUDA(cudaEventCreate(&r->ev1));
-    LD_CUDA(cudaEventCreate(&r->ev2));
   }
   if (r->dcap < dbytes) {
     if (r->dmem) { LD_CUDA(cudaStreamSynchronize(r->stream)); LD_CUDA(cudaFree(r->dmem)); r->dmem = nullptr; r->dcap = 0; }

@@ -87,7 +87,7 @@ struct Resources {
   size_t hcap = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
 void resources_release(Resources* r);

@@ -45,8 +45,10 @@ struct PruneArgs {
   unsigned long long expand;      // extensions of each, a power of the base
   unsigned long long run;         // consecutive extensions per thread, a power of the base up to it
   unsigned long long* list;       // surviving prefixes (evaluation: high indices)
-  unsigned long long* list_count; // their number
-  Slot* best;                     // evaluation: the best over its launches; then the high indices seen
+  unsigned long long* list_count; // their number; then a bound's first block's start and its last one's
+                                  // end (ns; all 0 before a bound)
+  Slot* best;                     // evaluation: the best over its launches; then the high indices seen,
+                                  // and the ns from the bounds' starts to the evaluations' ends
 };
 
 constexpr int kPruneThreads = 128;
@@ -240,6 +242,7 @@ template <int D, int WB, int WA>
 __global__ void __launch_bounds__(kPruneThreads) prefix_bound_kernel(const PruneArgs args) {
   using S = Shape<D, WB, WA>;
   extern __shared__ __align__(16) uint32_t smem[];
+  if (blockIdx.x == 0 && threadIdx.x == 0) args.list_count[1] = global_ns();
   stage<D, WB, WA>(args, smem, false);
   const TableArgs& ta = args.t;
   const int R = ta.R, k = ta.k, fw = ta.fw, nh = R - 1 - k;
@@ -300,6 +303,8 @@ __global__ void __launch_bounds__(kPruneThreads) prefix_bound_kernel(const Prune
       }
     }
   }
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(args.list_count + 2, global_ns());
 }
 
 // Evaluate the listed high indices: a thread per high index and part of the
@@ -354,7 +359,9 @@ __global__ void __launch_bounds__(kPruneThreads) prune_eval_kernel(const PruneAr
   if (grid_reduce(bv, bn, ta.red) && threadIdx.x == 0) {
     const Slot r = *ta.red.result;
     if (better(r.value, r.index, args.best->value, args.best->index)) *args.best = r;
-    *reinterpret_cast<unsigned long long*>(args.best + 1) += n;
+    unsigned long long* seen = reinterpret_cast<unsigned long long*>(args.best + 1);
+    seen[0] += n;
+    seen[1] += global_ns() - args.list_count[1];
   }
 }
 

@@ -2,6 +2,8 @@
 high indices, and the local search's two integer widths: the answers are those
 of the plain enumeration (itself checked against the oracle) and of the same
 moves made one by one in Python."""
+import time
+
 import numpy as np
 import pytest
 
@@ -46,6 +48,41 @@ def test_everything_survives(ld, rows, cols, d):
     sol, st = ld.solve_pruned(a, d, False, None, ld.options(prune_policy=1, enumerate_all=1))
     assert (sol.value, sol.gray_index) == (plain.value, plain.gray_index)
     assert st["highs_kept"] == st["highs_visited"] == st["highs_total"]
+
+
+@pytest.mark.parametrize("rows,cols", [(14, 16), (12, 64)])
+def test_reported_device_time_is_the_launches(ld, rows, cols):
+    """bound_ms and scan_ms hold the search's launches, not the host's waits and
+    the solve of the low rows between them, which alone takes longer than the
+    bound and the evaluation of one walk (two short launches)."""
+    a = _matrix(np.random.default_rng(rows * 100 + cols), rows, cols, 300)
+    vals, labs = ld.local_search(a, 1, False, n_random=16, seed=2)
+    lab, scan, norm = labs[int(np.argmax(vals))], [], []
+    for _ in range(20):
+        sol, st = ld.solve_pruned(a, 1, False, lab, ld.options(prune_policy=1))
+        assert st["pruned"] == 1 and sol.kernel_ms == pytest.approx(st["bound_ms"] + st["scan_ms"])
+        assert 0 < st["bound_ms"] and 0 < st["scan_ms"]
+        scan.append(st["scan_ms"])
+    low = np.concatenate([a[:st["low_rows"]], np.zeros((1, cols), np.int64)])
+    for _ in range(20):
+        t0 = time.perf_counter()
+        ld.solve_reduced(low, 1)
+        norm.append((time.perf_counter() - t0) * 1e3)
+    assert min(scan) < min(norm)
+
+
+@pytest.mark.parametrize("rows", [14, 33])
+def test_reported_upload_holds_the_levels(ld, rows):
+    """d = 2 uploads the prefix rows' column totals (16 words) for every level,
+    d = 1 the image alone, which has the same size."""
+    a = _matrix(np.random.default_rng(rows), rows, 16, "lowrank") * 100
+    sent = []
+    for d in (1, 2):
+        vals, labs = ld.local_search(a, d, False, n_random=16, seed=1)
+        sol, st = ld.solve_pruned(a, d, False, labs[int(np.argmax(vals))], ld.options(prune_policy=1))
+        assert st["pruned"] == 1
+        sent.append(sol.h2d_bytes)
+    assert sent[1] > sent[0] and (sent[1] - sent[0]) % 64 == 0
 
 
 def _climb(a, d, marg, lab):
