@@ -178,3 +178,30 @@ def test_inside_a_batch(ld, tune):
             with pytest.raises(ld.LdError) as e:
                 b.solve()
             assert e.value.status == 7 and "entry 0" in str(e.value)
+
+
+@pytest.mark.parametrize("d,cols,amp,seed,chunks", [(1, 17, 3, 24, 1), (1, 20, 3, 27, 2), (2, 10, 3, 24, 1), (2, 11, 3, 25, 2),
+                                                    (2, 15, 3, 29, 3), (3, 15, 2, 36, 1), (3, 15, 3, 36, 2), (3, 18, 3, 39, 3),
+                                                    (4, 17, 2, 45, 1), (4, 17, 3, 45, 2), (4, 17, 3, 17, 3)])
+def test_weights_above_one_in_every_number_of_chunks(ld, d, cols, amp, seed, chunks):
+    """Entries to +-2 and +-3: thresholds that share a feature, in tiles of one,
+    two and three chunks for every order (+-1 entries reach three chunks for d = 1
+    and 3 alone)."""
+    a = np.random.default_rng(seed).integers(-amp, amp + 1, size=(ROWS[d], cols)).astype(np.int64)
+    sol, desc = _solve(ld, a, d, False)
+    assert _chunks(desc) == chunks, desc
+    assert (sol.value, sol.gray_index) == O.enumerate_max(a, d, False), desc
+
+
+@pytest.mark.parametrize("d,cols", [(1, 40), (2, 24), (3, 30), (4, 21)])
+def test_every_low_labeling_of_a_block_ties(ld, d, cols):
+    """Rows of the table that are zero: all labelings of a block have its value,
+    and the block's first Gray index is the one reported."""
+    low = {1: 8, 2: 8, 3: 5, 4: 4}[d]
+    for seed in range(4):
+        a = np.random.default_rng(seed).choice(np.array([-1, 1], dtype=np.int64), size=(ROWS[d], cols))
+        a[:low] = 0
+        sol, desc = _solve(ld, a, d, False)
+        assert _tc(desc) > 0 and f" k={low} " in desc, desc
+        assert (sol.value, sol.gray_index) == O.enumerate_max(a, d, False), desc
+        assert sol.gray_index % (2 if d <= 2 else d) ** low == 0
