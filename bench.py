@@ -109,7 +109,7 @@ def issue_ops_per_labeling(desc: str, d: int, cols: int) -> tuple[int, str]:
     issue at half the ALU pipe's add/xor rate, so each costs 2 slots of the
     int32 add/xor peak.  The LM instances that add the marginal column
     linearly skip its word.  Wide kernel: the plain count.  Tensor-core form
-    (tc=): int8 tensor operations instead, against INT8_PEAK."""
+    (tc=): int8 tensor operations instead, against int8_peak."""
     f = dict(kv.split("=") for kv in desc.replace("int32 words", "int32_words")
              .replace("int8x4 words", "int8x4_words").split() if "=" in kv)
     if int(f.get("tc", 0)) > 0:
@@ -135,10 +135,17 @@ def issue_ops_per_labeling(desc: str, d: int, cols: int) -> tuple[int, str]:
     return ops_per_labeling(d, cols), "plain count (wide kernel)"
 
 
-# int8 tensor operations per second: products of 128 x 256 x 32 issued back to
-# back from tensor memory, 7800 multiply-adds per clock and SM (measured; 148
-# SMs at 1965 MHz).
-INT8_PEAK = 2 * 7800 * 148 * 1.965e9
+# int8 multiply-adds per clock and SM of products of 128 x 256 x 32 issued back to
+# back, the first operand in shared memory (as in tc_kernel) or in tensor memory.
+# A recorded constant, not measured in the run: a probe with a commit per 128
+# products gave 7700 on a B200 at 1965 MHz, the commits' 200 clocks taken out 7800.
+INT8_MACS = 7800
+
+
+def int8_peak(sms: int, sm_mhz: float) -> float:
+    """int8 tensor operations per second at an SM clock."""
+    return 2.0 * INT8_MACS * sms * sm_mhz * 1e6
+
 
 # DRAM traffic of one launch of the kernel that solves config 2, from the ncu
 # capture summarised in profiles/tc_kernel.md (dram__bytes_read.sum +
@@ -592,7 +599,13 @@ def run_ours(args) -> None:
         opl = ops_per_labeling(d, info["cols"])
         iopl, iwhat = issue_ops_per_labeling(desc, d, info["cols"])
         tensor = " tc=" in desc and not desc.endswith(" tc=0")
-        peak_ops = INT8_PEAK if tensor else ld.int32_peak(local)[0]
+        if tensor:
+            sms, mhz = torch.cuda.get_device_properties(local).multi_processor_count, clk["sm_mhz"] or 1965.0
+            peak_ops = int8_peak(sms, mhz)
+            peak_what = (f"{INT8_MACS} multiply-adds per clock and SM (a recorded constant) on {sms} SMs at {mhz:g} MHz"
+                         + (", the median SM clock of the timed region" if clk["sm_mhz"] else ", no clock sampled"))
+        else:
+            peak_ops, peak_what = ld.int32_peak(local)[0], "int32 add/xor microbenchmark measured in this run"
         # labelings the kernel computed a value for (d >= 3: the walks that
         # hold no smallest index of a label-permutation class are skipped)
         evaluated = int(sol.evaluated)
@@ -618,8 +631,7 @@ def run_ours(args) -> None:
                                           "x_peak": opl * rate / peak_ops},
                          "note": f"achieved = {iopl} {'int8 tensor operations' if tensor else 'int32 issue slots'} "
                                  f"per labeling ({iwhat}) x evaluated labelings/s; "
-                                 f"peak = {'128x256x32 products issued back to back, measured' if tensor else 'int32 add/xor microbenchmark measured in this run'}"
-                                 f"; plain_method "
+                                 f"peak = {peak_what}; plain_method "
                                  f"counts the {'3m' if d == 1 else '6m'} ops the plain enumeration spends per "
                                  f"labeling (m={info['cols']}), which the table decomposition avoids"},
             "e2e": {"value": e2e_value, "unit": "labelings/s", "h2d_bytes_per_step": h2d,

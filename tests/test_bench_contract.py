@@ -115,3 +115,9 @@ def test_issue_slots_of_the_column_split_count_real_columns(bench):
     d = ("table D=3 int32 words=0 int8x4 words=64 lin=0 pair=0 k=3 B=27 fw=0 walks=1 run=1 sym=5 "
          "blocks=1 tpb=128 smem=1 split=4 p16=1")
     assert bench.issue_ops_per_labeling(d, 3, 250)[0] == 2 * 3 * 63
+
+
+def test_int8_peak_follows_the_clock_and_the_device(bench):
+    assert bench.int8_peak(148, 1965.0) == pytest.approx(2 * 7800 * 148 * 1.965e9)
+    assert bench.int8_peak(74, 1310.0) == pytest.approx(bench.int8_peak(148, 1965.0) / 3)
+    assert bench.issue_ops_per_labeling("table D=1 int32 words=0 int8x4 words=0 half=0 tc=256", 1, 37)[0] == 512
