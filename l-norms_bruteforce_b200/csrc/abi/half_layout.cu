@@ -19,8 +19,32 @@ void half_pack(const int64_t* v, const int64_t* bias, int C, int W, int S, uint3
   }
 }
 
-bool half_layout(const int64_t* a, int R, int C, int d, int marginal, int k, int W, int S, HalfLayout* out) {
-  if (2 * W * S < C) return false;
+HalfSums::HalfSums(const int64_t* a, int R, int C, int d, int marginal, int k0, int k1)
+    : C(C), d(d), marginal(marginal), k0(k0), tot(C, 0), pos(C, 0), neg(C, 0), low_pos((size_t)(k1 - k0 + 1) * C),
+      low_neg((size_t)(k1 - k0 + 1) * C) {
+  for (int i = 0; i < R && fields; ++i) {
+    const int64_t* row = a + (size_t)i * C;
+    if (i >= k0 && i <= k1) low(i);
+    for (int c = 0; c < C; ++c) {
+      const int64_t v = row[c];
+      if (v > 65535 || v < -65535) fields = false;
+      tot[c] += v;
+      if (d == 1 || i < R - 1) (v < 0 ? neg : pos)[c] += v < 0 ? -v : v;
+    }
+  }
+  if (R <= k1) low(R);
+}
+
+void HalfSums::low(int k) {
+  std::copy(pos.begin(), pos.end(), low_pos.begin() + (size_t)(k - k0) * C);
+  std::copy(neg.begin(), neg.end(), low_neg.begin() + (size_t)(k - k0) * C);
+}
+
+bool half_layout(const HalfSums& sums, int k, int W, int S, HalfLayout* out) {
+  const int C = sums.C, d = sums.d, marginal = sums.marginal;
+  const int64_t* low_pos = sums.low_pos.data() + (size_t)(k - sums.k0) * C;
+  const int64_t* low_neg = sums.low_neg.data() + (size_t)(k - sums.k0) * C;
+  if (2 * W * S < C || !sums.fields) return false;
   out->W = W;
   out->S = S;
   out->beta.assign(C, 0);
@@ -32,14 +56,9 @@ bool half_layout(const int64_t* a, int R, int C, int d, int marginal, int k, int
     int64_t beta_sum = 0, st_min = 0, st_max = 0, st_any = 0;
     const int c0 = g * 2 * W, c1 = std::min(C, c0 + 2 * W);
     for (int c = c0; c < c1; ++c) {
-      int64_t hn = 0, hp = 0, ln = 0, lp = 0, low_sum = 0, tot = 0;   // negative / positive parts, high and low rows
-      for (int i = 0; i < R; ++i) {
-        const int64_t v = a[(size_t)i * C + c];
-        if (v > 65535 || v < -65535) return false;
-        tot += v;
-        if (i < k) { (v < 0 ? ln : lp) += v < 0 ? -v : v; low_sum += v; }
-        else if (d == 1 || i < R - 1) (v < 0 ? hn : hp) += v < 0 ? -v : v;
-      }
+      // negative / positive parts of the high and low rows
+      const int64_t lp = low_pos[c], ln = low_neg[c], hp = sums.pos[c] - lp, hn = sums.neg[c] - ln;
+      const int64_t low_sum = lp - ln, tot = sums.tot[c];
       // ranges of the register vectors and of the table vectors compared with them
       int64_t h_lo[3], h_hi[3], t_lo[3], t_hi[3];
       const int nv = d == 1 ? 1 : d;
@@ -74,6 +93,10 @@ bool half_layout(const int64_t* a, int R, int C, int d, int marginal, int k, int
     out->value_bias += (int)(2 * (low[0] + low[1] - q - beta_sum) - (st_any & 1));
   }
   return true;
+}
+
+bool half_layout(const int64_t* a, int R, int C, int d, int marginal, int k, int W, int S, HalfLayout* out) {
+  return half_layout(HalfSums(a, R, C, d, marginal, k, k), k, W, S, out);
 }
 
 }  // namespace ldsolve

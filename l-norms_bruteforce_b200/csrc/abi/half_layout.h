@@ -14,8 +14,21 @@ struct HalfLayout {
   int value_bias = 0;             // value = 2 Y - SH + value_bias (- the LM shift)
 };
 
+// A matrix's column sums by sign: of all rows a labeling moves (d = 1: the fixed
+// row too), and of the low ones alone for k = k0 .. k1 of them (at most R).
+struct HalfSums {
+  HalfSums(const int64_t* a, int R, int C, int d, int marginal, int k0, int k1);
+  int C, d, marginal, k0;
+  bool fields = true;                             // every entry fits a 16-bit field
+  std::vector<int64_t> tot, pos, neg;             // signed over all rows; positive, negative parts
+  std::vector<int64_t> low_pos, low_neg;          // (k - k0) x C + c
+ private:
+  void low(int k);
+};
+
 // Fills *out, or returns false when a column's values do not fit a 16-bit
 // field or a half of the packed accumulator could pass 65535.
+bool half_layout(const HalfSums& sums, int k, int W, int S, HalfLayout* out);
 bool half_layout(const int64_t* a, int R, int C, int d, int marginal, int k, int W, int S, HalfLayout* out);
 
 // Words of one stored vector over all slices: S x half_row_words(W).
