@@ -217,7 +217,8 @@ ld_status ld_solve_reduced_noalloc(const int64_t *mtx_as_vec, int32_t rows, int3
 /* ld_solve_reduced's.  `incumbent_labels` (rows-1 labels, may be NULL) is  */
 /* a labeling whose value the host recomputes.  d <= 3 inside the table     */
 /* kernel's range; other inputs fall back to the plain enumeration          */
-/* (stats->pruned = 0).                                                     */
+/* (stats->pruned = 0).  Working memory: up to 48 MB of prefix lists per    */
+/* device, kept for the next call.                                          */
 typedef struct {
     uint64_t walks_total, walks_kept;         /* top-row prefixes, and those not pruned */
     uint64_t highs_total, highs_visited, highs_kept;  /* high indices (blocks of `block` labelings) */

@@ -444,7 +444,7 @@ extern "C" ld_status ld_batch_create(int32_t count, const int64_t* const* mats, 
   };
 
   // autotuner: per class, the instance (plain or column-split), threads per
-  // CTA (64, 128, 256), walks per thread per chunk (1, 2, 4, 8; the chunk
+  // CTA (64, 128), walks per thread per chunk (1, 2, 4, 8; the chunk
   // holds threads x walks walks) and the persistent grid (half or all of the
   // occupancy limit), timed on one wave of the class's chunks from its
   // median matrix on and normalised per labeling.  Every candidate is timed

@@ -13,9 +13,9 @@
 // accumulators.  Thresholds u that no reachable H separates share a feature
 // (its weight counts them), those outside H's range need none; a +-1 or
 // -1/0/1 matrix needs about as many features per column as there are low
-// rows, 5 to 9.  The product costs (features / 61) clocks per labeling and SM
-// quarter, the 8-bit table kernel 2.3 per four columns: 37 columns with
-// marginals (208 features) 3.7 against 22 clocks.
+// rows, 5 to 9.  Per 32 labelings and SM quarter the product costs (features /
+// 61) clocks, the 8-bit table kernel 2.3 for four columns: 34 x 37 with
+// marginals (256 features) 4.2 against 22 clocks.
 //
 // One persistent CTA per SM, 18 warps:
 //   warps 8-15 (producers, two sets of four)  walk the high indices: H as
