@@ -156,7 +156,6 @@ __device__ __forceinline__ bool grid_reduce(long long v, unsigned long long n, c
   __shared__ bool s_last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int nwarps = (blockDim.x + 31) >> 5;
-  HostSlot* host = threadIdx.x == 0 ? host_slot(R) : nullptr;
   warp_best(v, n);
   if (lane == 0) { s_v[wid] = v; s_n[wid] = n; }
   __syncthreads();
@@ -168,7 +167,7 @@ __device__ __forceinline__ bool grid_reduce(long long v, unsigned long long n, c
       R.slots[blockIdx.x].value = v;
       R.slots[blockIdx.x].index = n;
       if (v != LLONG_MIN) atomicMax(R.gvalue, v);
-      if (host) atomicMin(start_word(R), block_clock());
+      if (host_slot(R)) atomicMin(start_word(R), block_clock());
       __threadfence();
       unsigned int done = atomicAdd(R.counter, 1u);
       s_last = (done == gridDim.x - 1);
@@ -194,7 +193,7 @@ __device__ __forceinline__ bool grid_reduce(long long v, unsigned long long n, c
     for (int w = 0; w < nwarps; ++w) if (s_n[w] < best) best = s_n[w];
     R.result->value = gmax;
     R.result->index = best;
-    if (host) *host = HostSlot{gmax, best, atomicExch(start_word(R), ULLONG_MAX), global_ns()};
+    if (HostSlot* host = host_slot(R)) *host = HostSlot{gmax, best, atomicExch(start_word(R), ULLONG_MAX), global_ns()};
     *R.gvalue = LLONG_MIN;
     *R.counter = 0u;
     if (R.work) *R.work = 0ull;   // every block has finished fetching walks
